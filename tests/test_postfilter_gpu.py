@@ -1,0 +1,31 @@
+"""GPU: the DC blocker's block scan against the recursion as written, in double."""
+import numpy as np
+import pytest
+
+from parallelfdtd_gb300 import postfilter as pf
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 511, 512, 513, 8191, 8192, 8193, 17000])
+@pytest.mark.parametrize("a", [0.995, 1.0, -0.7, 0.0, 1.0005])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_dc_block_equals_recursion(gpu, n, a, dtype):
+    """y[t] = x[t] - x[t-1] + a y[t-1] at sizes around a thread's samples, a
+    warp's and a tile's; |a| > 1 takes the serial kernel.  Each of the n sums
+    of the chain rounds to at most eps of the largest partial sum, and the scan
+    adds as many again, with the powers of a rounded on top: 4 n eps of the
+    largest value; float results round once more."""
+    x = np.random.default_rng(n).standard_normal((3, n)).astype(dtype)
+    want = np.zeros((3, n))
+    xp = yp = np.zeros(3)
+    for t in range(n):
+        yp = x[:, t].astype(np.float64) - xp + a * yp
+        xp = x[:, t].astype(np.float64)
+        want[:, t] = yp
+    got = pf.fir(x, np.array([1.0]), dc_coef=a)
+    assert got.dtype == dtype
+    tol = 4 * n * np.finfo(np.float64).eps * np.abs(want).max()
+    if dtype == np.float32:
+        tol = tol + np.finfo(np.float32).eps * np.abs(want)
+    assert np.all(np.abs(got.astype(np.float64) - want) <= tol)
