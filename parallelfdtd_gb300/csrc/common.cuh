@@ -180,6 +180,16 @@ struct GraphCache {
   int64_t launches = 0;  // kernels in one replay (counted while capturing)
 };
 
+// Bricks and inboxes of the resident run (resident.cu), planned once per domain.
+struct ResidentState {
+  bool planned = false, ok = false;
+  int brick[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  void* inbox = nullptr;     // face exchange words, zeroed when tags start over
+  int words = 0;             // of one brick's inbox half
+  size_t bytes = 0;
+  uint32_t tag = 1;          // of the next step
+};
+
 }  // namespace pfdtd
 
 // The opaque domain handle.
@@ -220,6 +230,7 @@ struct pfdtd_domain {
   int class_scheme = -1;
   int class_form = 0;        // update form the class table was built for
   int n_classes = 0;
+  int air_class = -1;        // a class of open air (loss-free, no missing neighbour)
   int cls_bytes = 1;
   void* d_cls = nullptr;     // per node class id (uint8 or uint16)
   // The class ids with every row padded to a multiple of 16 bytes, for the
@@ -288,6 +299,7 @@ struct pfdtd_domain {
   // loads in flight always keeps its own 2 s bound
   uint64_t wait_ns = 2000000000ull;
   pfdtd::TmaState tma;
+  pfdtd::ResidentState resident;
 
   // temporal blocking (stencil_tb.cu): requested depth (0 off) and the
   // geometry check it depends on, cached per class build
@@ -339,6 +351,10 @@ int tma_tile_count();
 int launch_update_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 int launch_iwb_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 bool uses_tma(const pfdtd_domain* d);
+// Implemented in resident.cu
+bool resident_usable(pfdtd_domain* d);
+int launch_resident(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64_t rec_ld,
+                    int64_t inject_end, cudaStream_t s);
 // Implemented in stencil_tb.cu
 int tb_usable(const pfdtd_domain* d, std::string* why);
 int launch_tb(pfdtd_domain* d, void* rec_out, int64_t rec_ld, int64_t inject_end, cudaStream_t s);

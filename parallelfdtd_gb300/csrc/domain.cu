@@ -221,12 +221,53 @@ int prepare_run(pfdtd_domain* d) {
   return PFDTD_OK;
 }
 
+// Steps of one resident launch when nobody asks between chunks.
+constexpr int64_t kResidentChunk = 8192;
+
+// enqueue_run for a grid that stays on the SMs (resident.cu): launches of
+// `chunk` steps instead of graphs of single steps.
+template <typename F>
+int enqueue_resident(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool* stopped,
+                     int64_t* steps_queued, int64_t chunk) {
+  cudaStream_t s = d->stream;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  PFDTD_CK(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
+  PFDTD_CK(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
+  int rc = PFDTD_OK;
+  int64_t done = 0;
+  *stopped = false;
+  for (int64_t k = 0; done < steps && rc == PFDTD_OK; ++k) {
+    if (k >= 2) {
+      cudaError_t e = cudaEventSynchronize(ev[k % 2]);
+      int perr = 0;
+      if (e == cudaSuccess) e = cudaMemcpy(&perr, d->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) { rc = cuda_fail(e, "resident run", __FILE__, __LINE__); break; }
+      // an expired wait is reported by check_pipeline after the sync
+      if (perr || between((k - 1) * chunk)) { *stopped = true; break; }
+    }
+    const int64_t n = std::min(chunk, steps - done);
+    rc = launch_resident(d, done, n, rec_out, steps, steps, s);
+    if (rc) break;
+    done += n;
+    cudaError_t e = cudaEventRecord(ev[k % 2], s);
+    if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventRecord", __FILE__, __LINE__);
+  }
+  cudaEventDestroy(ev[0]);
+  cudaEventDestroy(ev[1]);
+  *steps_queued = done;
+  return rc;
+}
+
 // Queue `steps` steps recording into rec_out (device, [n_rec * steps]).
 // Between chunks `between(k_done)` may be called after waiting for chunk
 // completion; it returns non-zero to stop.
 template <typename F>
 int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool* stopped,
-                int64_t* steps_queued, bool poll = true) {
+                int64_t* steps_queued, bool poll = true, int64_t resident_chunk = kResidentChunk) {
+  // (asynchronous runs share the GPU with other domains' runs and keep to
+  // single steps: a resident launch would hold every SM for its whole length)
+  if (poll && resident_usable(d))
+    return enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, resident_chunk);
   cudaStream_t s = d->stream;
   PFDTD_CK(cudaMemsetAsync(d->d_step, 0, sizeof(int64_t), s));
   if (int rc0 = launch_dif_init(d, s)) return rc0;
@@ -279,11 +320,20 @@ int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool
   return rc;
 }
 
-// Queue `n` steps continuing from the device step counter, without host
-// waits: chunk graphs for whole chunks, then blocked launches and single
-// steps.  rec_ld / inject_end as in enqueue_run (the run's step count).
-int enqueue_steps(pfdtd_domain* d, int64_t n, void* rec_out, int64_t rec_ld, int64_t inject_end) {
+// Queue `n` steps continuing from step `at` (also the device step counter),
+// without host waits: resident launches, or chunk graphs for whole chunks, then
+// blocked launches and single steps.  rec_ld / inject_end as in enqueue_run
+// (the run's step count).
+int enqueue_steps(pfdtd_domain* d, int64_t at, int64_t n, void* rec_out, int64_t rec_ld,
+                  int64_t inject_end) {
   cudaStream_t s = d->stream;
+  if (resident_usable(d)) {
+    for (int64_t done = 0; done < n; done += kResidentChunk)
+      if (int rc = launch_resident(d, at + done, std::min(kResidentChunk, n - done), rec_out, rec_ld,
+                                   inject_end, s))
+        return rc;
+    return PFDTD_OK;
+  }
   const int tb = tb_active(d) ? d->tb_depth : 0;
   const int64_t chunk = tb ? kChunkTb : kChunk;
   int64_t done = 0;
@@ -420,7 +470,7 @@ int pfdtd_destroy(pfdtd_domain* d) {
                   d->d_ctab, d->d_src_idx, d->d_src_mode, d->d_src_samples, d->d_rec_idx,
                   d->d_step, d->d_rec_out, d->d_err, d->d_dif_list, d->d_dif_tab,
                   d->d_dif_state, d->d_iwb_mask, d->d_iwb_code, d->d_iwb_sw,
-                  d->d_iwb_closure, d->d_iwb_closure_dif, d->d_cls_tma};
+                  d->d_iwb_closure, d->d_iwb_closure_dif, d->d_cls_tma, d->resident.inbox};
   for (void* p : ptrs)
     d->release(p);
   if (d->stream) cudaStreamDestroy(d->stream);
@@ -679,7 +729,8 @@ int pfdtd_run(pfdtd_domain* d, int64_t steps, void* out, pfdtd_interrupt_fn inte
   };
   bool stopped = false;
   int64_t queued = 0;
-  rc = enqueue_run(d, steps, d->d_rec_out, between, &stopped, &queued);
+  rc = enqueue_run(d, steps, d->d_rec_out, between, &stopped, &queued, true,
+                   interrupt_cb || progress_cb ? kChunk : kResidentChunk);
   if (rc) return rc;
   // Rows of receivers outside the grid are left untouched (kernels3d.cu:184-191).
   const size_t row = (size_t)steps * d->arith_size();
@@ -766,7 +817,7 @@ int pfdtd_run_captures(pfdtd_domain* d, int64_t steps, void* out, int n_cap,
   int64_t at = 0;
   for (int k = 0; k < n_cap && rc == PFDTD_OK; ++k) {
     const int i = order[k];
-    rc = enqueue_steps(d, cap_step[i] - at, d->d_rec_out, steps, steps);
+    rc = enqueue_steps(d, at, cap_step[i] - at, d->d_rec_out, steps, steps);
     at = cap_step[i];
     if (rc) break;
     float* dp = p_out && p_out[i] ? sp + offset[i] : nullptr;
@@ -778,9 +829,9 @@ int pfdtd_run_captures(pfdtd_domain* d, int64_t steps, void* out, int n_cap,
     if (e == cudaSuccess && dq) e = cudaMemcpyAsync(pos_out[i], dq, size[i], cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) rc = cuda_fail(e, "capture copy", __FILE__, __LINE__);
   }
-  if (rc == PFDTD_OK) rc = enqueue_steps(d, steps - at, d->d_rec_out, steps, steps);
-  // record the receivers of the last step; never inject
-  if (rc == PFDTD_OK && steps > 0) rc = launch_io(d, d->cur_field(), d->d_rec_out, steps, 0, s);
+  if (rc == PFDTD_OK) rc = enqueue_steps(d, at, steps - at, d->d_rec_out, steps, steps);
+  // record the receivers of the last step (resident launches have); never inject
+  if (rc == PFDTD_OK && steps > 0 && !resident_usable(d)) rc = launch_io(d, d->cur_field(), d->d_rec_out, steps, 0, s);
   if (rc == PFDTD_OK) {
     const size_t row = (size_t)steps * d->arith_size();
     for (int r = 0; r < d->n_rec && rc == PFDTD_OK && steps > 0; ++r)

@@ -384,6 +384,20 @@ int launch_io(pfdtd_domain* d, void* cur, void* rec_out, int64_t rec_ld, int64_t
   return fail(PFDTD_ERR_UNSUPPORTED, "unknown precision");
 }
 
+// The class of open air: all neighbours present (forward K = 6, centred no
+// boundary axis), inside, its loss factors exactly 1 (air nodes of material 0
+// first); -1 if there is none.
+template <typename A>
+static int find_air(int scheme, const std::vector<uint16_t>& keys, const std::vector<uint8_t>& tab) {
+  const unsigned pos = scheme == PFDTD_SRL ? 0x80u : 0x86u;
+  const size_t n = keys.size();
+  const A* a = (const A*)tab.data();
+  const A c = scheme == PFDTD_SRL ? (A)-1 : (A)1;
+  for (size_t i = 0; i < n; ++i)
+    if ((keys[i] >> 8) == pos && a[i] == (A)1 && a[2 * n + i] == c) return (int)i;
+  return -1;
+}
+
 // Build the class ids and the coefficient table for the domain's current
 // scheme, quirks, parameters and materials.
 int build_classes(pfdtd_domain* d) {
@@ -493,6 +507,9 @@ int build_classes(pfdtd_domain* d) {
   }
   PFDTD_CK(cudaStreamSynchronize(s));
   d->n_classes = n_classes;
+  d->air_class = scheme == PFDTD_IWB            ? -1
+                 : d->precision == PFDTD_F64 ? find_air<double>(scheme, keys, tab)
+                                                : find_air<float>(scheme, keys, tab);
   d->class_scheme = scheme;
   d->class_form = form;
   rc = build_dif(d, keys, tab);

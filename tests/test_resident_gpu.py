@@ -1,0 +1,146 @@
+"""GPU: runs whose grid stays on the SMs, against the CPU oracle bit for bit.
+
+Sizes lie around the brick splits: a brick's x vector of 4, bricks cut short on
+each axis, one brick, one node of air, long and flat rooms, and the largest
+number of planes a thread holds.  Fields start from random values, planes 0 and
+Z-1 (never updated) included, and the step counts are odd, so that both buffers
+of a halo exchange and both field roles are used."""
+import numpy as np
+import pytest
+
+from parallelfdtd_gb300 import _lib as L
+from parallelfdtd_gb300 import rooms
+from parallelfdtd_gb300.domain import Domain, default_params
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def O(built):
+    from oracle import oracle
+    return oracle
+
+
+def _values(rng, n, prec):
+    v = rng.uniform(-1.0, 1.0, n).astype(np.float32)
+    if prec == "bf16":
+        return (v.view(np.uint32) >> 16).astype(np.uint16)
+    return v.astype({"f32": np.float32, "f64": np.float64, "f16": np.float16}[prec])
+
+
+def _as_float(v):
+    """Field values as numbers (BF16 comes as bit patterns): a zero on an x or y
+    face may differ in sign, as in the temporally blocked runs."""
+    return (v.astype(np.uint32) << 16).view(np.float32) if v.dtype == np.uint16 else v
+
+
+def _check(O, dims, prec, scheme, steps, form="reference", runs=1, progress=None, captures=()):
+    room = rooms.boxes_room(dims, n_boxes=3 if min(dims) > 16 else 0, edge=(4, 9), n_materials=5,
+                            seed=sum(dims))
+    rng = np.random.default_rng(steps)
+    inside = np.flatnonzero(room.bid)
+    some_air = inside.size > 0
+    if not some_air:  # the closed room of 3 nodes across is all solid
+        inside = np.array([room.flat(1, 1, 1)])
+    pick = rng.choice(inside, 7)
+    src, rec = [room.coords(int(i)) for i in pick[:3]], [room.coords(int(i)) for i in pick[3:]]
+    src.append(src[0])  # a second source on one node: order matters
+    types = [1, 0, 1, 1]
+    pulses = rng.uniform(-1.0, 1.0, (4, steps))
+    P0, Pp0 = _values(rng, room.n_nodes, prec), _values(rng, room.n_nodes, prec)
+    with Domain(dims, prec) as d:
+        d.set_scheme(scheme)
+        d.set_voxels(room.bid, room.mat, centred=scheme == "centred")
+        d.set_materials(room.admittance)
+        d.set_params()
+        if form != "reference":
+            d.set_update_form(form)
+        d.set_sources(src, types, pulses)
+        d.set_receivers(rec)
+        for _ in range(runs):  # the same start again: exchange tags go on
+            d.upload_field(L.FIELD_CURRENT, P0)
+            d.upload_field(L.FIELD_PAST, Pp0)
+            if captures:
+                got, slices = d.run_captures(steps, [(c, 0, dims[2] // 2) for c in captures])
+            else:
+                got, _, st = d.run(steps, progress=progress)
+                assert st == 0
+            P, Pp = d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)
+            if runs > 1 and steps % 2:
+                d.flip()  # the same buffers' roles as at first
+    pos, mat = O.encode_nodes(room.bid, room.mat, scheme == "centred")
+
+    def oracle(n):
+        return O.run(pos, mat, dims, room.admittance, default_params(),
+                     [room.flat(*p) for p in src], types, pulses[:, :n], [room.flat(*p) for p in rec], n,
+                     scheme=2 if scheme == "centred" else 0, double=prec == "f64",
+                     storage=prec if prec in ("f16", "bf16") else None, P0=P0, Pp0=Pp0, form=form)
+    want, rP, rPp = oracle(steps)
+    assert (np.abs(want).max() > 0) == some_air
+    assert np.array_equal(got, want)
+    assert np.array_equal(_as_float(P), _as_float(rP))
+    assert np.array_equal(_as_float(Pp), _as_float(rPp))
+    if captures:
+        X, Y, _ = dims
+        for c, (p, _) in zip(captures, slices):
+            z = oracle(c)[1].reshape(dims[2], Y, X)[dims[2] // 2]
+            assert np.array_equal(p, z.astype(np.float32)), c
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4), (5, 3, 7), (33, 17, 9), (64, 64, 64), (130, 31, 40),
+                                  (21, 260, 12), (16, 18, 300), (301, 40, 33), (128, 120, 130)])
+def test_sizes(gpu, O, dims):
+    _check(O, dims, "f32", "forward", 61)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64", "f16", "bf16"])
+@pytest.mark.parametrize("scheme", ["forward", "centred"])
+@pytest.mark.parametrize("dims", [(40, 37, 26), (90, 70, 61)])
+def test_types(gpu, O, dims, prec, scheme):
+    _check(O, dims, prec, scheme, 23)
+
+
+def test_difference_form(gpu, O):
+    _check(O, (75, 42, 31), "f32", "forward", 41, form="difference")
+
+
+def test_largest_double(gpu, O):
+    _check(O, (128, 100, 98), "f64", "forward", 21)
+
+
+def test_repeated_run(gpu, O):
+    _check(O, (52, 36, 45), "f32", "forward", 33, runs=3)
+
+
+def test_chunks_with_progress(gpu, O):
+    """With a callback the run is split into short launches: 120 steps in three."""
+    seen = []
+    _check(O, (52, 36, 45), "f32", "forward", 120, progress=lambda s, n, t: seen.append(s))
+    assert seen == [0, 100]
+
+
+def test_captures(gpu, O):
+    _check(O, (52, 36, 45), "f32", "forward", 31, captures=(0, 4, 5, 31))
+
+
+@pytest.mark.parametrize("place", [(0, 20, 10), (30, 20, 0)])
+def test_other_rooms_take_the_general_path(gpu, O, place):
+    """Inside nodes on an x face, or a source on plane 0: not resident, and as
+    the oracle has it."""
+    room = rooms.shoebox((48, 40, 36), seed=3)
+    bid = room.bid.copy().reshape(36, 40, 48)
+    if place[0] == 0:
+        bid[5:30, 8:30, 0] = 27
+    pulse = rooms.gaussian_pulse(40, 3.0)[None]
+    with Domain(room.dims) as d:
+        d.set_voxels(bid.reshape(-1), room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([place], [1], pulse)
+        d.set_receivers([(24, 20, 18)])
+        got, _, _ = d.run(40)
+        P = d.download_field(L.FIELD_CURRENT)
+    pos, mat = O.encode_nodes(bid.reshape(-1), room.mat, False)
+    want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(),
+                        [room.flat(*place)], [1], pulse, [room.flat(24, 20, 18)], 40)
+    assert np.array_equal(got, want) and np.array_equal(P, rP)
