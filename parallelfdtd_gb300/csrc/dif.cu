@@ -111,6 +111,7 @@ __global__ void k_dif_update(const int64_t* __restrict__ list, int64_t n, int ks
   using A = typename Store<S>::A;
   using R = Rn<A>;
   using Sto = Store<S>;
+  step_ready();
   // X, XY count field elements; the x neighbour is K elements away.
   const int64_t ks = (int64_t)1 << kshift;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
@@ -240,6 +241,7 @@ k_iwb_closure(const ClosureRec* __restrict__ recs, int64_t n, ClassTab<float> ta
               float* __restrict__ iwb_sw, const int32_t* __restrict__ dif_slot,
               const float* __restrict__ dtab, float* __restrict__ dstate) {
   using Sto = Store<S>;
+  step_ready();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const ClosureRec r = recs[k];
@@ -350,27 +352,24 @@ int launch_dif_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int g = grid_for(n);
   const float* iwb_sw =
       (d->class_scheme == PFDTD_IWB && d->d_iwb_sw && uses_tma(d)) ? d->d_iwb_sw : nullptr;
+  auto launch = [&](auto kernel) {
+    return launch_plain(kernel, dim3(g), dim3(256), 0, s, d->d_dif_list, n, d->kshift, d->d_cls,
+                              d->cls_bytes, (const A*)d->d_dif_tab, (const S*)cur, (S*)past,
+                              (A*)d->d_dif_state, XE, XYE, l2, cpos, d->d_iwb_mask, iwb_sw);
+  };
+  cudaError_t e;
   switch (d->class_scheme) {
     case PFDTD_SRL:
-      k_dif_update<S, 1><<<g, 256, 0, s>>>(d->d_dif_list, n, d->kshift, d->d_cls, d->cls_bytes,
-                                           (const A*)d->d_dif_tab, (const S*)cur, (S*)past,
-                                           (A*)d->d_dif_state, XE, XYE, l2, cpos,
-                                           d->d_iwb_mask, iwb_sw);
+      e = launch(k_dif_update<S, 1>);
       break;
     case PFDTD_IWB:
-      k_dif_update<S, 2><<<g, 256, 0, s>>>(d->d_dif_list, n, d->kshift, d->d_cls, d->cls_bytes,
-                                           (const A*)d->d_dif_tab, (const S*)cur, (S*)past,
-                                           (A*)d->d_dif_state, XE, XYE, l2, cpos,
-                                           d->d_iwb_mask, iwb_sw);
+      e = launch(k_dif_update<S, 2>);
       break;
     default:
-      k_dif_update<S, 0><<<g, 256, 0, s>>>(d->d_dif_list, n, d->kshift, d->d_cls, d->cls_bytes,
-                                           (const A*)d->d_dif_tab, (const S*)cur, (S*)past,
-                                           (A*)d->d_dif_state, XE, XYE, l2, cpos,
-                                           d->d_iwb_mask, iwb_sw);
+      e = launch(k_dif_update<S, 0>);
   }
+  PFDTD_CK(e);
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 
@@ -519,13 +518,12 @@ int launch_closure_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t 
                       (const float*)(ctab + 2 * (size_t)nc * 4),
                       (const uint32_t*)(ctab + 3 * (size_t)nc * 4), nc};
   const bool fuse = iwb_closure_fuses_dif(d);
-  k_iwb_closure<S><<<grid_for(n), 256, 0, s>>>(
-      (const ClosureRec*)d->d_iwb_closure, n, tab, (const S*)cur, (S*)past, d->X, d->XY,
-      (float)d->params[1], (d->n_dif > 0 && !fuse) ? d->d_iwb_sw : nullptr,
-      fuse ? d->d_iwb_closure_dif : nullptr, fuse ? (const float*)d->d_dif_tab : nullptr,
-      fuse ? (float*)d->d_dif_state : nullptr);
+  PFDTD_CK(launch_plain(
+      k_iwb_closure<S>, dim3(grid_for(n)), dim3(256), 0, s, (const ClosureRec*)d->d_iwb_closure, n, tab,
+      (const S*)cur, (S*)past, d->X, d->XY, (float)d->params[1],
+      (d->n_dif > 0 && !fuse) ? d->d_iwb_sw : nullptr, fuse ? d->d_iwb_closure_dif : nullptr,
+      fuse ? (const float*)d->d_dif_tab : nullptr, fuse ? (float*)d->d_dif_state : nullptr));
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 

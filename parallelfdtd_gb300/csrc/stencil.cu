@@ -47,6 +47,8 @@ k_update_zmarch(const C* __restrict__ cls, const S* __restrict__ P, S* __restric
     }
     __syncthreads();
   }
+  step_wait();
+  step_ready();
   // X and XY count field elements (nodes times ks fields); ks is the element
   // distance of the x neighbour.
   const int x = blockIdx.x * kBX + threadIdx.x;
@@ -120,6 +122,8 @@ k_update_iwb(const C* __restrict__ cls, const uint32_t* __restrict__ mask,
   using A = typename Store<S>::A;
   using R = Rn<A>;
   using St = Store<S>;
+  step_wait();
+  step_ready();
   const int x = blockIdx.x * kBX + threadIdx.x;
   const int y = blockIdx.y * kBY + threadIdx.y;
   const int z0 = 1 + blockIdx.z * zc;
@@ -218,8 +222,14 @@ __global__ void k_iwb_geometry(const uint8_t* __restrict__ pos, int64_t N, int64
 // Between two updates: record receivers from the current field for the step
 // just finished (kernels3d.cu:164-173), then inject this step's source
 // samples into the current field in source order (kernels3d.cu:93-104).
+//
+// The kernel is one chain of dependent loads between two updates: 3.4 us of
+// a step (step counter, index, field value, sample one after the other, each
+// source by itself).  Now everything but the field is read before the update
+// it follows has ended (the update starts it after the last k_step_io's end, so
+// the counter stands), and after the wait one round trip to L2 is left.
 template <typename S>
-__global__ void k_step_io(S* __restrict__ cur, int64_t* __restrict__ d_step, int n_rec,
+__global__ void k_step_io(S* cur, volatile int64_t* d_step, int n_rec,
                           const int64_t* __restrict__ rec_idx,
                           typename Store<S>::A* __restrict__ rec_out,
                           int64_t rec_ld, int n_src, const int64_t* __restrict__ src_idx,
@@ -228,29 +238,52 @@ __global__ void k_step_io(S* __restrict__ cur, int64_t* __restrict__ d_step, int
                           int64_t inject_end, int advance) {
   using A = typename Store<S>::A;
   using St = Store<S>;
+  const int t = threadIdx.x;
   const int64_t n = *d_step;
-  if (n > 0 && rec_out != nullptr) {
-    for (int r = threadIdx.x; r < n_rec; r += blockDim.x) {
+  const bool inject = n < inject_end && n < n_samples;
+  // one warp injects, 32 sources at a time
+  int64_t node = -1;
+  int mode = 0;
+  A sample = (A)0;
+  auto fetch = [&](int k) {
+    node = k < n_src ? src_idx[k] : -1;
+    mode = k < n_src ? src_mode[k] : 0;
+    sample = k < n_src ? samples[(int64_t)k * n_samples + n] : (A)0;
+  };
+  if (t < 32 && inject) fetch(t);
+  const bool record = n > 0 && rec_out != nullptr && n - 1 < rec_ld;
+  const int64_t mine = record && t < n_rec ? rec_idx[t] : -1;
+  step_ready();
+  step_wait();
+  if (record) {
+    if (mine >= 0) rec_out[(int64_t)t * rec_ld + (n - 1)] = St::load(cur[mine]);
+    for (int r = t + blockDim.x; r < n_rec; r += blockDim.x) {
       const int64_t i = rec_idx[r];
-      if (i >= 0 && n - 1 < rec_ld) rec_out[(int64_t)r * rec_ld + (n - 1)] = St::load(cur[i]);
+      if (i >= 0) rec_out[(int64_t)r * rec_ld + (n - 1)] = St::load(cur[i]);
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (n < inject_end && n < n_samples) {
-      for (int k = 0; k < n_src; ++k) {
-        const int64_t i = src_idx[k];
-        if (i < 0) continue;
-        const A v = samples[(int64_t)k * n_samples + n];
-        if (src_mode[k] == 0)
-          cur[i] = St::store(v);
-        else
-          cur[i] = St::store(Rn<A>::add(St::load(cur[i]), v));
+  if (t < 32 && inject) {
+    for (int base = 0; base < n_src; base += 32) {
+      if (base > 0) fetch(base + t);
+      // sources on one node: its first lane applies them all, in order
+      const unsigned same = __match_any_sync(0xffffffffu, (unsigned long long)node);
+      const bool first = node >= 0 && __ffs(same) - 1 == t;
+      A v = first ? St::load(cur[node]) : (A)0;
+      unsigned left = same;
+      while (__any_sync(0xffffffffu, first && left != 0)) {
+        const int j = left != 0 ? __ffs(left) - 1 : t;
+        const A s = __shfl_sync(0xffffffffu, sample, j);
+        const int m = __shfl_sync(0xffffffffu, mode, j);
+        if (first && left != 0) v = St::load(St::store(m == 0 ? s : Rn<A>::add(v, s)));
+        left &= left - 1;
       }
+      if (first) cur[node] = St::store(v);
+      __syncwarp();
     }
-    // A temporally blocked update that follows advances by its depth.
-    *d_step = n + advance;
   }
+  // A temporally blocked update that follows advances by its depth.
+  if (t == 0) *d_step = n + advance;
 }
 
 // Presence of (pos, mat) keys over the updated planes z = 1..Z-2.
@@ -287,11 +320,10 @@ int launch_update_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  k_update_zmarch<S, C, SCHEME><<<dim3(gx, gy, gz), dim3(kBX, kBY), 0, s>>>(
-      (const C*)d->d_cls, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y, d->XY * d->K,
-      (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift);
+  PFDTD_CK(launch_step_kernel(k_update_zmarch<S, C, SCHEME>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
+                              (const C*)d->d_cls, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y,
+                              d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift));
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 
@@ -312,11 +344,11 @@ int launch_iwb_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  k_update_iwb<S, C><<<dim3(gx, gy, gz), dim3(kBX, kBY), 0, s>>>(
-      (const C*)d->d_cls, d->d_iwb_mask, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y,
-      d->XY * d->K, (int)(d->Z - 1), (int)zc, d->K, d->kshift, (A)d->params[1]);
+  PFDTD_CK(launch_step_kernel(k_update_iwb<S, C>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
+                              (const C*)d->d_cls, d->d_iwb_mask, (const S*)cur, (S*)past, tab, (int)XE,
+                              (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, d->K, d->kshift,
+                              (A)d->params[1]));
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 
@@ -343,12 +375,11 @@ int launch_io_t(pfdtd_domain* d, void* cur, void* rec_out, int64_t rec_ld, int64
                 cudaStream_t s, int advance) {
   using A = typename Store<S>::A;
   const int threads = std::max(32, std::min(1024, ((d->n_rec + 31) / 32) * 32));
-  k_step_io<S><<<1, threads, 0, s>>>((S*)cur, d->d_step, d->n_rec, d->d_rec_idx, (A*)rec_out,
-                                    rec_ld, d->n_src, d->d_src_idx, d->d_src_mode,
-                                    (const A*)d->d_src_samples, d->n_samples, inject_end,
-                                    advance);
+  PFDTD_CK(launch_step_kernel(k_step_io<S>, dim3(1), dim3(threads), 0, s, (S*)cur, (volatile int64_t*)d->d_step,
+                              d->n_rec, d->d_rec_idx, (A*)rec_out, rec_ld, d->n_src, d->d_src_idx,
+                              d->d_src_mode, (const A*)d->d_src_samples, d->n_samples, inject_end,
+                              advance));
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 

@@ -422,9 +422,6 @@ k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant_
   unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   __shared__ PackedCoef<A> stab[kSmemTab ? 256 : 1];
 
-  // A launch after one whose pipeline failed does nothing: the run is
-  // already invalid and the host reports it.
-  if (*(volatile int*)err) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * TY;
   const int z0 = 1 + blockIdx.z * zc;
@@ -448,6 +445,11 @@ k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant_
       stab[i] = PackedCoef<A>{tab.a[i], tab.b[i], tab.c[i], tab.pos[i]};
   }
   __syncthreads();
+  step_wait();
+  step_ready();
+  // A launch after one whose pipeline failed does nothing: the run is
+  // already invalid and the host reports it.
+  if (*(volatile int*)err) return;
   if (nplanes <= 0) return;
   const int K = nplanes + 2;  // loads: planes z0-1 .. z1 of P^n
 
@@ -978,13 +980,12 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  k_update_tma<S, C, SCHEME, Lay, BATCHED><<<dim3(gx, gy, gz), Lay::THREADS, Lay::SMEM, s>>>(
-      ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur,
-      (S*)past, tab, (int)XE, (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc,
-      (A)d->params[1], d->d_err, d->kshift, SCHEME == 3 ? d->d_iwb_sw : nullptr, -0.0f,
-      d->wait_ns);
+  PFDTD_CK(launch_step_kernel(
+      k_update_tma<S, C, SCHEME, Lay, BATCHED>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
+      ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur, (S*)past,
+      tab, (int)XE, (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->d_err,
+      d->kshift, SCHEME == 3 ? d->d_iwb_sw : nullptr, -0.0f, d->wait_ns));
   count_launch();
-  PFDTD_CK(cudaGetLastError());
   return PFDTD_OK;
 }
 
