@@ -308,7 +308,8 @@ int pfdtd_fetch_receivers(pfdtd_domain* d, void* out);
 
 /* Update kernel variant: 0 automatic (the TMA-pipelined kernel when the
  * field rows are 16-byte aligned: X * fields * element size a multiple of 16;
- * class-id rows that are not are read from a padded copy), 1 the
+ * class-id rows that are not are read from a padded copy; a single FP64 field
+ * takes the z-march kernel), 1 the
  * register z-marching kernel, 2 the TMA kernel.  pfdtd_get_kernel reports the
  * variant the next launch will use (1 or 2, or 3 when the temporally blocked
  * kernel of pfdtd_set_temporal_block will run). */

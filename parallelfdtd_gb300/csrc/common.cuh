@@ -117,6 +117,48 @@ __device__ __forceinline__ void iwb_sums(const A (&m)[3][3][3], A& s1, A& s2, A&
   s3 = R::add(iwb_c2(m[0]), iwb_c2(m[2]));
 }
 
+// The FP64 7-point update of a node of any class.  Not inlined: as a branch of
+// the update kernels the compiler would predicate it, and a predicated-off FP64
+// operation still takes its 76 cycles of the scheduler's FP64 unit.
+template <int SCHEME>
+__device__ __noinline__ double srl_node_f64(double pc, double pm, double pn, double xm, double xp,
+                                            double ym, double yp, double pp, double a, double b,
+                                            double c, uint32_t cp, double l2) {
+  using R = Rn<double>;
+  if constexpr (SCHEME == 1) {
+    const double dx = (double)(cp & 1u), dy = (double)((cp >> 1) & 1u), dz = (double)((cp >> 2) & 1u);
+    const double bx = (cp & 0x10u) ? xp : xm;
+    const double by = (cp & 0x20u) ? yp : ym;
+    const double bz = (cp & 0x40u) ? pm : pn;
+    const double sb6 = R::add(R::add(R::mul(bx, dx), R::mul(by, dy)), R::mul(bz, dz));
+    const double s7 = R::add(R::add(R::add(R::add(R::add(R::add(xm, xp), ym), yp), pn), pm), sb6);
+    return R::mul(a, R::add(R::sub(R::mul(s7, l2), R::mul(b, pc)), R::mul(c, pp)));
+  } else {
+    const double s6 = R::add(R::add(R::add(R::add(R::add(pn, pm), yp), ym), xp), xm);
+    return R::mul(a, R::sub(R::add(R::mul(b, pc), R::mul(l2, s6)), R::mul(c, pp)));
+  }
+}
+// The same in open air (a = 1, c = +-1, no boundary axis) without the products
+// by 1 and, centred, without the boundary neighbours times 0: equal while those
+// are finite.
+template <int SCHEME>
+__device__ __forceinline__ double srl_air_f64(double pc, double pm, double pn, double xm, double xp,
+                                              double ym, double yp, double pp, double b, double l2) {
+  using R = Rn<double>;
+  if constexpr (SCHEME == 1) {
+    const double s6 = R::add(R::add(R::add(R::add(R::add(xm, xp), ym), yp), pn), pm);
+    return R::sub(R::sub(R::mul(s6, l2), R::mul(b, pc)), pp);
+  } else {
+    const double s6 = R::add(R::add(R::add(R::add(R::add(pn, pm), yp), ym), xp), xm);
+    return R::sub(R::add(R::mul(b, pc), R::mul(l2, s6)), pp);
+  }
+}
+
+// Whether a value is infinite or not a number (integer test).
+__device__ __forceinline__ bool not_finite(double v) {
+  return ((unsigned)__double2hiint(v) & 0x7FF00000u) == 0x7FF00000u;
+}
+
 // Storage type -> arithmetic type.
 template <typename S> struct Store;
 template <> struct Store<float> {

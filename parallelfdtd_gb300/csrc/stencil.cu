@@ -30,7 +30,7 @@ template <typename S, typename C, int SCHEME>
 __global__ void __launch_bounds__(kBX * kBY)
 k_update_zmarch(const C* __restrict__ cls, const S* __restrict__ P, S* __restrict__ Pp,
                 ClassTab<typename Store<S>::A> tab, int X, int Y, int64_t XY, int z_last,
-                int zc, typename Store<S>::A l2, int ks, int kshift) {
+                int zc, typename Store<S>::A l2, int ks, int kshift, unsigned air) {
   using A = typename Store<S>::A;
   using R = Rn<A>;
   using St = Store<S>;
@@ -75,7 +75,16 @@ k_update_zmarch(const C* __restrict__ cls, const S* __restrict__ P, S* __restric
       ca = __ldg(tab.a + c); cb = __ldg(tab.b + c); cc = __ldg(tab.c + c); cp = __ldg(tab.pos + c);
     }
     A out;
-    if (SCHEME == 0 || SCHEME == 4) {
+    if constexpr (sizeof(A) == 8) {
+      // FP64 operations bound this kernel: a warp in open air leaves out its
+      // exact products by 1 and, centred, the zero of its boundary neighbours
+      // (see k_update_tma)
+      const bool plain = c == air && !(SCHEME == 1 && (not_finite(xm) || not_finite(ym) || not_finite(pn)));
+      if (__all_sync(__activemask(), plain))
+        out = srl_air_f64<SCHEME>(pc, pm, pn, xm, xp, ym, yp, pp, cb, l2);
+      else
+        out = srl_node_f64<SCHEME>(pc, pm, pn, xm, xp, ym, yp, pp, ca, cb, cc, cp, l2);
+    } else if (SCHEME == 0 || SCHEME == 4) {
       // S = P[z+1] + P[z-1] + P[y+1] + P[y-1] + P[x+1] + P[x-1]  (kernels3d.cu:525)
       const A s6 = R::add(R::add(R::add(R::add(R::add(pn, pm), yp), ym), xp), xm);
       if (SCHEME == 4) {
@@ -322,7 +331,8 @@ int launch_update_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
   PFDTD_CK(launch_step_kernel(k_update_zmarch<S, C, SCHEME>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
                               (const C*)d->d_cls, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y,
-                              d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift));
+                              d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift,
+                              (unsigned)d->air_class));
   count_launch();
   return PFDTD_OK;
 }

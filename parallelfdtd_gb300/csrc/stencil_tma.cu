@@ -407,7 +407,7 @@ k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant_
              S* __restrict__ Pp, ClassTab<typename Store<S>::A> tab, int X, int Y, int64_t XY,
              int z_last, int zc, typename Store<S>::A l2, int* __restrict__ err, int kshift = 0,
              float* __restrict__ iwb_sw = nullptr, float nzf = -0.0f,
-             uint64_t wait_ns = kWaitLimitNs) {
+             uint64_t wait_ns = kWaitLimitNs, unsigned air = 0xFFFFFFFFu) {
   using A = typename Store<S>::A;
   using R = Rn<A>;
   using St = Store<S>;
@@ -650,6 +650,44 @@ k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant_
             const __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
             res[2 * h] = __low2bfloat16(t);
             res[2 * h + 1] = __high2bfloat16(t);
+          }
+        }
+        stgv<VEC>(Pp + idx, res);
+      } else if constexpr (sizeof(A) == 8 && SCHEME != 3) {
+        // FP64: an SM issues 1.7 operations a cycle, which bounds this kernel,
+        // so a warp whose nodes are all open air (class `air`: a = 1, c = +-1,
+        // no boundary axis) leaves out the products by 1 and, centred, the
+        // boundary neighbours times 0, which add a zero unless one of them is
+        // not finite.  (512 x 384 x 256, forward: 1080 -> 970 us.)
+        A xm[VEC], xp[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          xm[e] = BATCHED ? St::load(vxm.v[e]) : (e == 0 ? left : fc[e > 0 ? e - 1 : 0]);
+          xp[e] = BATCHED ? St::load(vxp.v[e]) : (e == VEC - 1 ? right : fc[e < VEC - 1 ? e + 1 : e]);
+        }
+        auto coef = [&](unsigned c) -> PackedCoef<A> {
+          if (kSmemTab) return stab[c];
+          return PackedCoef<A>{__ldg(tab.a + c), __ldg(tab.b + c), __ldg(tab.c + c), __ldg(tab.pos + c)};
+        };
+        bool plain = true;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          plain = plain && cid[e] == air;
+          if constexpr (SCHEME == 1)
+            plain = plain && !not_finite(xm[e]) && !not_finite(vym.v[e]) && !not_finite(fn[e]);
+        }
+        S res[VEC];
+        if (__all_sync(__activemask(), plain)) {
+          const A b = coef(air).b;
+#pragma unroll
+          for (int e = 0; e < VEC; ++e)
+            res[e] = srl_air_f64<SCHEME>(fc[e], fm[e], fn[e], xm[e], xp[e], vym.v[e], vyp.v[e], vpp.v[e], b, l2);
+        } else {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) {
+            const PackedCoef<A> k = coef(cid[e]);
+            res[e] = srl_node_f64<SCHEME>(fc[e], fm[e], fn[e], xm[e], xp[e], vym.v[e], vyp.v[e], vpp.v[e],
+                                          k.a, k.b, k.c, k.pos, l2);
           }
         }
         stgv<VEC>(Pp + idx, res);
@@ -956,7 +994,12 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int gx = (int)((XE + kTX - 1) / kTX);
   const int gy = (int)((d->Y + Lay::TY - 1) / Lay::TY);
   // z-chunks: several per tile so that the grid fills the machine in whole
-  // waves of (SMs x resident CTAs), each chunk at least 16 planes long.
+  // waves of (SMs x resident CTAs), each chunk at least 16 planes long.  FP64 is
+  // bound by its operations, which a chunk's two more planes of loads do not
+  // add to: chunks of 4 planes or more, for an even share of the work
+  // (100 x 90 x 80, 8 fields: 195 -> 135 us).
+  constexpr int kMinPlanes = sizeof(A) == 8 ? 4 : 16;
+  constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : 2.0;
   const int64_t per_sm =
       occ > 0
           ? occ
@@ -965,12 +1008,12 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int64_t tiles = (int64_t)gx * gy;
   int64_t best_c = 1;
   double best = 1e30;
-  for (int64_t c = 1; c <= std::max<int64_t>(1, nz / 16); ++c) {
+  for (int64_t c = 1; c <= std::max<int64_t>(1, nz / kMinPlanes); ++c) {
     const int64_t ctas = tiles * c;
     const int64_t waves = (ctas + resident - 1) / resident;
     const double eff = (double)ctas / (double)(waves * resident);  // wave fill
     const double zlen = (double)nz / (double)c;
-    const double cost = 1.0 / eff * (1.0 + 2.0 / zlen);
+    const double cost = 1.0 / eff * (1.0 + kMorePlanes / zlen);
     if (cost < best - 1e-9) { best = cost; best_c = c; }
   }
   const int64_t zc = (nz + best_c - 1) / best_c;
@@ -984,7 +1027,7 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
       k_update_tma<S, C, SCHEME, Lay, BATCHED>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
       ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur, (S*)past,
       tab, (int)XE, (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->d_err,
-      d->kshift, SCHEME == 3 ? d->d_iwb_sw : nullptr, -0.0f, d->wait_ns));
+      d->kshift, SCHEME == 3 ? d->d_iwb_sw : nullptr, -0.0f, d->wait_ns, (unsigned)d->air_class));
   count_launch();
   return PFDTD_OK;
 }
@@ -1228,6 +1271,12 @@ bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
 bool uses_tma(const pfdtd_domain* d) {
   if (d->kernel_variant == PFDTD_KERNEL_ZMARCH || !tma_supported(d)) return false;
   if (d->class_scheme == PFDTD_IWB) return d->K == 1 && d->precision != PFDTD_F64;
+  // FP64 operations bound a single FP64 field: the z-march kernel, with 64
+  // warps on an SM and small blocks to share them evenly, keeps the FP64 units
+  // busier than the stage ring's 12 warps (forward 121 against 163 us on
+  // 256 x 192 x 128, 905 against 970 on 512 x 384 x 256; centred 169 / 290 and
+  // 1087 / 1278).
+  if (d->precision == PFDTD_F64 && d->K == 1 && d->kernel_variant == PFDTD_KERNEL_AUTO) return false;
   return true;
 }
 
@@ -1247,6 +1296,10 @@ bool tma_supported(const pfdtd_domain* d) {
   // (rows of class ids that are not 16-byte aligned are read from a padded
   // copy, d_cls_tma)
   if ((d->X * (int64_t)d->esize) % 16 != 0) return false;
+  // A consumer thread stores whole vectors of 4, so a row is a whole number of
+  // them (for FP64 aligned rows alone would allow X = 2 mod 4, whose last
+  // vector runs into the next row).
+  if (d->X * d->K % 4 != 0) return false;
   if (d->Y * d->Z >= ((int64_t)1 << 31)) return false;
   return encode_fn() != nullptr;
 }
