@@ -363,6 +363,10 @@ struct pfdtd_domain {
   int64_t* d_step = nullptr;
   void* d_rec_out = nullptr;
   size_t rec_out_bytes = 0;
+  // receiver values and error flag of pfdtd_step: host memory that the device
+  // writes (allocated by the first step)
+  void* step_out_h = nullptr;
+  size_t step_out_bytes = 0;
   cudaStream_t stream = nullptr;
   pfdtd::GraphCache graph;
   int past_step_direction = 1;
@@ -412,7 +416,8 @@ namespace pfdtd {
 // Implemented in stencil.cu
 int launch_update(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 int launch_io(pfdtd_domain* d, void* cur, void* rec_out, int64_t rec_ld, int64_t inject_end,
-              cudaStream_t s, int advance = 1);
+              cudaStream_t s, int advance = 1, int64_t step = -1);
+int launch_step_out(pfdtd_domain* d, const void* cur, cudaStream_t s);
 int build_classes(pfdtd_domain* d);
 // noalloc.cu: puts the no-allocation capture's scratch on `device` (current).
 int noalloc_prepare(int device);

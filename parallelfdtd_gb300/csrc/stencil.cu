@@ -244,11 +244,11 @@ __global__ void k_step_io(S* cur, volatile int64_t* d_step, int n_rec,
                           int64_t rec_ld, int n_src, const int64_t* __restrict__ src_idx,
                           const int32_t* __restrict__ src_mode,
                           const typename Store<S>::A* __restrict__ samples, int64_t n_samples,
-                          int64_t inject_end, int advance) {
+                          int64_t inject_end, int advance, int64_t step) {
   using A = typename Store<S>::A;
   using St = Store<S>;
   const int t = threadIdx.x;
-  const int64_t n = *d_step;
+  const int64_t n = step >= 0 ? step : *d_step;  // the step index may come from the host
   const bool inject = n < inject_end && n < n_samples;
   // one warp injects, 32 sources at a time
   int64_t node = -1;
@@ -293,6 +293,21 @@ __global__ void k_step_io(S* cur, volatile int64_t* d_step, int n_rec,
   }
   // A temporally blocked update that follows advances by its depth.
   if (t == 0) *d_step = n + advance;
+}
+
+// Receivers of the current field and the pipeline error flag into host memory
+// (the flag in the first 16 bytes), for pfdtd_step.
+template <typename S>
+__global__ void k_step_out(const S* cur, int n_rec, const int64_t* __restrict__ rec_idx,
+                           const int* err, void* host) {
+  using A = typename Store<S>::A;
+  step_wait();
+  if (threadIdx.x == 0) *(volatile int*)host = *err;
+  A* out = (A*)((char*)host + 16);
+  for (int r = threadIdx.x; r < n_rec; r += blockDim.x) {
+    const int64_t i = rec_idx[r];
+    if (i >= 0) out[r] = Store<S>::load(cur[i]);
+  }
 }
 
 // Presence of (pos, mat) keys over the updated planes z = 1..Z-2.
@@ -382,13 +397,13 @@ int launch_update_s(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s
 
 template <typename S>
 int launch_io_t(pfdtd_domain* d, void* cur, void* rec_out, int64_t rec_ld, int64_t inject_end,
-                cudaStream_t s, int advance) {
+                cudaStream_t s, int advance, int64_t step) {
   using A = typename Store<S>::A;
   const int threads = std::max(32, std::min(1024, ((d->n_rec + 31) / 32) * 32));
   PFDTD_CK(launch_step_kernel(k_step_io<S>, dim3(1), dim3(threads), 0, s, (S*)cur, (volatile int64_t*)d->d_step,
                               d->n_rec, d->d_rec_idx, (A*)rec_out, rec_ld, d->n_src, d->d_src_idx,
                               d->d_src_mode, (const A*)d->d_src_samples, d->n_samples, inject_end,
-                              advance));
+                              advance, step));
   count_launch();
   return PFDTD_OK;
 }
@@ -414,13 +429,31 @@ int launch_update(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) 
 }
 
 int launch_io(pfdtd_domain* d, void* cur, void* rec_out, int64_t rec_ld, int64_t inject_end,
-              cudaStream_t s, int advance) {
+              cudaStream_t s, int advance, int64_t step) {
   switch (d->precision) {
-    case PFDTD_F32: return launch_io_t<float>(d, cur, rec_out, rec_ld, inject_end, s, advance);
-    case PFDTD_F64: return launch_io_t<double>(d, cur, rec_out, rec_ld, inject_end, s, advance);
-    case PFDTD_F16: return launch_io_t<__half>(d, cur, rec_out, rec_ld, inject_end, s, advance);
+    case PFDTD_F32: return launch_io_t<float>(d, cur, rec_out, rec_ld, inject_end, s, advance, step);
+    case PFDTD_F64: return launch_io_t<double>(d, cur, rec_out, rec_ld, inject_end, s, advance, step);
+    case PFDTD_F16: return launch_io_t<__half>(d, cur, rec_out, rec_ld, inject_end, s, advance, step);
     case PFDTD_BF16:
-      return launch_io_t<__nv_bfloat16>(d, cur, rec_out, rec_ld, inject_end, s, advance);
+      return launch_io_t<__nv_bfloat16>(d, cur, rec_out, rec_ld, inject_end, s, advance, step);
+  }
+  return fail(PFDTD_ERR_UNSUPPORTED, "unknown precision");
+}
+
+template <typename S>
+static int launch_step_out_t(pfdtd_domain* d, const void* cur, cudaStream_t s) {
+  PFDTD_CK(launch_step_kernel(k_step_out<S>, dim3(1), dim3(std::max(32, std::min(1024, (d->n_rec + 31) / 32 * 32))),
+                              0, s, (const S*)cur, d->n_rec, d->d_rec_idx, (const int*)d->d_err, d->step_out_h));
+  count_launch();
+  return PFDTD_OK;
+}
+
+int launch_step_out(pfdtd_domain* d, const void* cur, cudaStream_t s) {
+  switch (d->precision) {
+    case PFDTD_F32: return launch_step_out_t<float>(d, cur, s);
+    case PFDTD_F64: return launch_step_out_t<double>(d, cur, s);
+    case PFDTD_F16: return launch_step_out_t<__half>(d, cur, s);
+    case PFDTD_BF16: return launch_step_out_t<__nv_bfloat16>(d, cur, s);
   }
   return fail(PFDTD_ERR_UNSUPPORTED, "unknown precision");
 }

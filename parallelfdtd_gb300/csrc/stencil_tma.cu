@@ -994,12 +994,14 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int gx = (int)((XE + kTX - 1) / kTX);
   const int gy = (int)((d->Y + Lay::TY - 1) / Lay::TY);
   // z-chunks: several per tile so that the grid fills the machine in whole
-  // waves of (SMs x resident CTAs), each chunk at least 16 planes long.  FP64 is
-  // bound by its operations, which a chunk's two more planes of loads do not
-  // add to: chunks of 4 planes or more, for an even share of the work
+  // waves of (SMs x resident CTAs), each chunk at least 4 planes long.  A
+  // chunk costs the two more planes that it loads and the time until its
+  // first stages arrive, about two planes' more (chunks of 16 planes or more
+  // left small rooms to a few CTAs: 10 us an update on 48 x 40 x 36, 3.9
+  // now).  FP64 is bound by its operations, which the loads do not add to
   // (100 x 90 x 80, 8 fields: 195 -> 135 us).
-  constexpr int kMinPlanes = sizeof(A) == 8 ? 4 : 16;
-  constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : 2.0;
+  constexpr int kMinPlanes = 4;
+  constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : 4.0;
   const int64_t per_sm =
       occ > 0
           ? occ
