@@ -306,11 +306,12 @@ int pfdtd_host_free(void* ptr);
 int pfdtd_query(pfdtd_domain* d, int* done);
 int pfdtd_fetch_receivers(pfdtd_domain* d, void* out);
 
-/* Update kernel variant: 0 automatic (the TMA-pipelined kernel when the
- * field rows are 16-byte aligned: X * fields * element size a multiple of 16;
- * class-id rows that are not are read from a padded copy; a single FP64 field
- * takes the z-march kernel), 1 the
- * register z-marching kernel, 2 the TMA kernel.  pfdtd_get_kernel reports the
+/* Update kernel variant: 0 automatic (a bulk-copy pipelined kernel: TMA tiles
+ * when the field rows are 16-byte aligned, X * fields * element size a multiple
+ * of 16, class-id rows that are not being read from a padded copy; runs of flat
+ * indices for other FP32 and 16-bit rooms with the 7-point schemes, and for
+ * large ones; a single FP64 field takes the z-march kernel), 1 the
+ * register z-marching kernel, 2 the pipelined kernels.  pfdtd_get_kernel reports the
  * variant the next launch will use (1 or 2, or 3 when the temporally blocked
  * kernel of pfdtd_set_temporal_block will run). */
 #define PFDTD_KERNEL_AUTO 0

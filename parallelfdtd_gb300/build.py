@@ -22,7 +22,8 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libpfdtd.so")
 
-CUDA_SOURCES = ["stencil.cu", "stencil_tma.cu", "resident.cu", "stencil_tb.cu", "stencil_tb_f32.cu",
+CUDA_SOURCES = ["stencil.cu", "stencil_tma.cu", "stencil_flat.cu", "resident.cu",
+                "stencil_tb.cu", "stencil_tb_f32.cu",
                 "stencil_tb_f16.cu", "stencil_tb_bf16.cu", "dif.cu", "domain.cu", "setup.cu",
                 "noalloc.cu", "voxelize.cu", "postfilter.cu"]
 CXX_SOURCES = [

@@ -440,6 +440,10 @@ int tma_tile_count();
 int launch_update_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 int launch_iwb_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 bool uses_tma(const pfdtd_domain* d);
+// Implemented in stencil_flat.cu
+bool flat_usable(const pfdtd_domain* d);
+int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
+bool prefers_flat(const pfdtd_domain* d);  // stencil_tma.cu
 // Implemented in resident.cu
 bool resident_usable(pfdtd_domain* d);
 int launch_resident(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64_t rec_ld,

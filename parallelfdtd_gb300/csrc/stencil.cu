@@ -416,9 +416,11 @@ int eval_class_coefs(int precision, int scheme, int form, int quirks, const doub
                      const std::vector<uint16_t>& keys, std::vector<uint8_t>& out_tab);
 
 int launch_update(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
-  if (uses_tma(d))
-    return d->class_scheme == PFDTD_IWB ? launch_iwb_tma(d, cur, past, s)
-                                        : launch_update_tma(d, cur, past, s);
+  if (uses_tma(d)) {
+    if (d->class_scheme == PFDTD_IWB) return launch_iwb_tma(d, cur, past, s);
+    return prefers_flat(d) ? launch_update_flat(d, cur, past, s) : launch_update_tma(d, cur, past, s);
+  }
+  if (flat_usable(d)) return launch_update_flat(d, cur, past, s);
   switch (d->precision) {
     case PFDTD_F32: return launch_update_s<float>(d, cur, past, s);
     case PFDTD_F64: return launch_update_s<double>(d, cur, past, s);

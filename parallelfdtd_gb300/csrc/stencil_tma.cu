@@ -24,6 +24,7 @@
 // error flag, stops issuing loads, waits (bounded) for the loads already in
 // flight and returns.
 #include "common.cuh"
+#include "mbar.cuh"
 
 #include <cuda.h>
 
@@ -37,8 +38,6 @@ namespace pfdtd {
 namespace {
 
 constexpr int kVec = 4;             // consecutive x elements per consumer thread (default)
-constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per wait, far above any real wait
-
 
 // Per-class coefficients packed for one 16-byte (float) or 32-byte (double)
 // shared-memory load per node.
@@ -85,80 +84,6 @@ struct Layout {
   static_assert(CONSUMER_WARPS * 32 * VEC == TX * TY, "consumer mapping");
   static_assert(PW <= 256 && (PW * (int)sizeof(S)) % 16 == 0, "TMA box row");
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Non-blocking test of the phase with the given parity.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// The waiting part of mbar_wait.  A bound under 1 ms (a watchdog set short)
-// polls without blocking and reads the clock at every poll, since a blocking
-// try_wait may itself sleep longer than such a bound; a longer bound blocks
-// in try_wait and reads the clock every 256 polls.
-__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-  const uint64_t t0 = global_ns();
-  if (limit_ns < 1000000ull) {
-    while (!mbar_test(bar, parity))
-      if (global_ns() - t0 > limit_ns) return false;
-    return true;
-  }
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try(bar, parity)) return true;
-    if ((i & 255) == 0 && global_ns() - t0 > limit_ns) return false;
-  }
-}
-
-// Wait for the phase with the given parity, for at most limit_ns; false on
-// expiry.  The common case in a streaming consumer, a phase already complete,
-// costs one non-blocking test.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
-                                          uint64_t limit_ns = kWaitLimitNs) {
-  if (mbar_test(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, limit_ns);
-}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y,
                                             uint32_t bar) {
@@ -1267,6 +1192,21 @@ bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
   // tile shapes 0..5 run the closure inside the streaming kernel
   return d->class_scheme == PFDTD_IWB && d->n_dif > 0 && d->iwb_closure_ready &&
          d->d_iwb_closure_dif != nullptr && uses_tma(d) && !(d->tma_tile >= 0 && d->tma_tile <= 5);
+}
+
+// Whether a room that the tiled kernel takes runs faster by flat runs
+// (stencil_flat.cu).  Measured, us an update, tiles / runs, FP32: forward 8 M nodes and more
+// (256^3 36.9 / 34.0, 512 x 384 x 256 99.9 / 95.8; 240 x 200 x 160 15.6 / 16.3), and
+// from 3 M where 256-wide tiles do not cover the rows (160^3 11.2 / 9.7, 320 x 240 x
+// 200 38.1 / 30.5, 128 x 150 x 150 of 2.9 M 7.6 / 7.8); centred only the latter
+// (384 x 320 x 256 74.7 / 71.2, 512 x 384 x 256 106 / 110); 16-bit fields, whose
+// tiles carry 8 nodes a thread, where only 64-wide tiles fit (160^3 11.9 / 10.4,
+// 384 x 320 x 256 41.0 / 56.9).
+bool prefers_flat(const pfdtd_domain* d) {
+  if (d->kernel_variant != PFDTD_KERNEL_AUTO || d->tma_tile >= 0 || d->K != 1) return false;
+  if (d->N < 3000000 || !flat_usable(d)) return false;
+  if (d->precision != PFDTD_F32) return auto_tile16(d) == 0;
+  return auto_tile(d) != 6 || (d->class_scheme != PFDTD_SRL && d->N >= 8000000);
 }
 
 // Whether the next update runs a TMA kernel (7-point or IWB).
