@@ -343,6 +343,10 @@ struct pfdtd_domain {
   // the closure pass also applies the DIF update (no separate DIF pass)
   int32_t* d_iwb_closure_dif = nullptr;
   bool iwb_closure_ready = false;
+  // IWB: every class has a = 0 outside the room, a = c = 1 and b = iwb_open_b
+  // inside without a closed neighbour
+  bool iwb_open = false;
+  float iwb_open_b = 0.f;
   int64_t class_version = 0;
 
   // sources / receivers
@@ -442,6 +446,7 @@ int launch_iwb_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s)
 bool uses_tma(const pfdtd_domain* d);
 // Implemented in stencil_flat.cu
 bool flat_usable(const pfdtd_domain* d);
+bool iwb_flat(const pfdtd_domain* d);
 int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 bool prefers_flat(const pfdtd_domain* d);  // stencil_tma.cu
 // Implemented in resident.cu

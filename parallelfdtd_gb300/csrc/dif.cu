@@ -351,7 +351,7 @@ int launch_dif_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int64_t XE = d->X * d->K, XYE = d->XY * d->K;
   const int g = grid_for(n);
   const float* iwb_sw =
-      (d->class_scheme == PFDTD_IWB && d->d_iwb_sw && uses_tma(d)) ? d->d_iwb_sw : nullptr;
+      (d->class_scheme == PFDTD_IWB && d->d_iwb_sw && (uses_tma(d) || iwb_flat(d))) ? d->d_iwb_sw : nullptr;
   auto launch = [&](auto kernel) {
     return launch_plain(kernel, dim3(g), dim3(256), 0, s, d->d_dif_list, n, d->kshift, d->d_cls,
                               d->cls_bytes, (const A*)d->d_dif_tab, (const S*)cur, (S*)past,

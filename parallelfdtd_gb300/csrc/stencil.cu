@@ -416,11 +416,12 @@ int eval_class_coefs(int precision, int scheme, int form, int quirks, const doub
                      const std::vector<uint16_t>& keys, std::vector<uint8_t>& out_tab);
 
 int launch_update(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
+  if (iwb_flat(d)) return launch_update_flat(d, cur, past, s);
   if (uses_tma(d)) {
     if (d->class_scheme == PFDTD_IWB) return launch_iwb_tma(d, cur, past, s);
     return prefers_flat(d) ? launch_update_flat(d, cur, past, s) : launch_update_tma(d, cur, past, s);
   }
-  if (flat_usable(d)) return launch_update_flat(d, cur, past, s);
+  if (d->class_scheme != PFDTD_IWB && flat_usable(d)) return launch_update_flat(d, cur, past, s);
   switch (d->precision) {
     case PFDTD_F32: return launch_update_s<float>(d, cur, past, s);
     case PFDTD_F64: return launch_update_s<double>(d, cur, past, s);
@@ -472,6 +473,23 @@ static int find_air(int scheme, const std::vector<uint16_t>& keys, const std::ve
   for (size_t i = 0; i < n; ++i)
     if ((keys[i] >> 8) == pos && a[i] == (A)1 && a[2 * n + i] == c) return (int)i;
   return -1;
+}
+
+// Whether the IWB classes outside the room and without closed neighbours (codes
+// 0 and 1) have the coefficients these codes stand for; a material that is not
+// finite makes others.
+static bool iwb_open_classes(const std::vector<uint16_t>& keys, const std::vector<uint8_t>& tab, float* b) {
+  const size_t n = keys.size();
+  const float* a = (const float*)tab.data();
+  *b = 0.f;
+  for (size_t i = 0; i < n; ++i) {
+    const unsigned code = keys[i] >> 8;
+    if (code == 0 && a[i] != 0.f) return false;
+    if (code != 1) continue;
+    if (a[i] != 1.f || a[2 * n + i] != 1.f) return false;
+    *b = a[n + i];
+  }
+  return true;
 }
 
 // Build the class ids and the coefficient table for the domain's current
@@ -586,6 +604,8 @@ int build_classes(pfdtd_domain* d) {
   d->air_class = scheme == PFDTD_IWB            ? -1
                  : d->precision == PFDTD_F64 ? find_air<double>(scheme, keys, tab)
                                                 : find_air<float>(scheme, keys, tab);
+  d->iwb_open = scheme == PFDTD_IWB && d->precision != PFDTD_F64 &&
+                iwb_open_classes(keys, tab, &d->iwb_open_b);
   d->class_scheme = scheme;
   d->class_form = form;
   rc = build_dif(d, keys, tab);

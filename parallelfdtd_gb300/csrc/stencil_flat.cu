@@ -43,11 +43,12 @@ struct alignas(16) Coef { float a, b, c; uint32_t pos; };
 
 __host__ __device__ inline int round128(int b) { return (b + 127) / 128 * 128; }
 
-// Bytes of a stage's three pieces, for rows of XE elements of es bytes.
+// Bytes of a stage's three pieces: elements of es bytes, `halo` more of P^n on
+// either side of the run.
 struct Stage { int past, cls, bytes; };  // offsets of P^{n-1} and class ids, size
-__host__ __device__ inline Stage stage_of(int XE, int es, int cs, int kshift) {
+__host__ __device__ inline Stage stage_of(int halo, int es, int cs, int kshift) {
   Stage s;
-  s.past = round128((kRange + 2 * XE) * es + 32);
+  s.past = round128((kRange + 2 * halo) * es + 32);
   s.cls = s.past + round128(kRange * es + 32);
   s.bytes = s.cls + round128((kRange >> kshift) * cs + 32);
   return s;
@@ -75,6 +76,44 @@ __device__ __forceinline__ void copy_piece(unsigned char* dst, const T* base, in
 // Where element `first` lies in the copied piece.
 template <typename T> __device__ __forceinline__ int remainder_of(int64_t first) {
   return (int)(first & (16 / (int64_t)sizeof(T) - 1));
+}
+
+// The producer thread: stage k receives `halo` elements around the run of P^n
+// plane z0-1+k and, from k = 2 on, the run of P^{n-1} and the class ids of plane
+// z0+k-2.  Every wait is bounded; on expiry it raises the error and abort flags,
+// and every copy in flight has landed before it returns.
+template <typename S, typename C>
+__device__ __forceinline__ void produce(unsigned char* smem, const Stage& lay, uint32_t full,
+                                        uint32_t empty, int* abort_flag, const S* P, const S* past,
+                                        const C* cls, int halo, int64_t XY, int64_t s0, int n, int z0,
+                                        int loads, int stages, int ks, int kshift, int* err,
+                                        uint64_t wait_ns) {
+  int issued = 0;
+  for (int k = 0; k < loads; ++k) {
+    const int slot = k % stages;
+    if (k >= stages && !mbar_wait(empty + 8 * slot, (uint32_t)((k / stages - 1) & 1), wait_ns)) {
+      atomicExch(err, 1);
+      *(volatile int*)abort_flag = 1;
+      break;
+    }
+    if (*(volatile int*)abort_flag) break;
+    unsigned char* st = smem + (size_t)slot * lay.bytes;
+    const uint32_t bar = full + 8 * slot;
+    const int64_t fp = (int64_t)(z0 - 1 + k) * XY + s0 - halo;
+    const int64_t fq = (int64_t)(z0 + k - 2) * XY + s0;
+    uint32_t bytes = piece_bytes<S>(fp, n + 2 * halo);
+    const int nc = (n + ks - 1) >> kshift;
+    if (k >= 2) bytes += piece_bytes<S>(fq, n) + piece_bytes<C>(fq >> kshift, nc);
+    mbar_expect_tx(bar, bytes);
+    copy_piece<S>(st, P, fp, n + 2 * halo, bar);
+    if (k >= 2) {
+      copy_piece<S>(st + lay.past, past, fq, n, bar);
+      copy_piece<C>(st + lay.cls, cls, fq >> kshift, nc, bar);
+    }
+    issued = k + 1;
+  }
+  for (int k = max(0, issued - stages); k < issued; ++k)
+    mbar_wait(full + 8 * (k % stages), (uint32_t)((k / stages) & 1));
 }
 
 template <typename S, typename C, int SCHEME>
@@ -114,38 +153,11 @@ k_update_flat(const S* __restrict__ P, S* __restrict__ Pp, const S* __restrict__
   step_ready();
   if (*(volatile int*)err) return;
   if (nplanes <= 0) return;
-  const int loads = nplanes + 2;
 
-  if (t >= kConsumers) {  // producer
-    if (lane != 0) return;
-    int issued = 0;
-    for (int k = 0; k < loads; ++k) {
-      const int slot = k % stages;
-      if (k >= stages &&
-          !mbar_wait(empty + 8 * slot, (uint32_t)((k / stages - 1) & 1), wait_ns)) {
-        atomicExch(err, 1);
-        *(volatile int*)&abort_flag = 1;
-        break;
-      }
-      if (*(volatile int*)&abort_flag) break;
-      unsigned char* st = smem + (size_t)slot * lay.bytes;
-      const uint32_t bar = full + 8 * slot;
-      const int64_t fp = (int64_t)(z0 - 1 + k) * XY + s0 - XE;
-      const int64_t fq = (int64_t)(z0 + k - 2) * XY + s0;
-      uint32_t bytes = piece_bytes<S>(fp, n + 2 * XE);
-      const int nc = (n + ks - 1) >> kshift;
-      if (k >= 2) bytes += piece_bytes<S>(fq, n) + piece_bytes<C>(fq >> kshift, nc);
-      mbar_expect_tx(bar, bytes);
-      copy_piece<S>(st, P, fp, n + 2 * XE, bar);
-      if (k >= 2) {
-        copy_piece<S>(st + lay.past, past, fq, n, bar);
-        copy_piece<C>(st + lay.cls, cls, fq >> kshift, nc, bar);
-      }
-      issued = k + 1;
-    }
-    // every copy in flight has landed before the CTA may end
-    for (int k = max(0, issued - stages); k < issued; ++k)
-      mbar_wait(full + 8 * (k % stages), (uint32_t)((k / stages) & 1));
+  if (t >= kConsumers) {
+    if (lane == 0)
+      produce<S, C>(smem, lay, full, empty, &abort_flag, P, past, cls, XE, XY, s0, n, z0, nplanes + 2,
+                    stages, ks, kshift, err, wait_ns);
     return;
   }
 
@@ -254,28 +266,170 @@ k_update_flat(const S* __restrict__ P, S* __restrict__ Pp, const S* __restrict__
   }
 }
 
+// IWB 27-point update by runs (no counterpart in the reference), one field per
+// node: every node takes the open sums here, and a node with a closed neighbour
+// (class flag bit 30) keeps P^{n-1} for the closure pass (k_iwb_closure,
+// dif.cu), as in the tiled kernel without masks.
+//
+// The in-plane sums (iwb_sums) of plane z+1 are made once, from nine values of
+// the stage; of planes z and z-1 the thread keeps what planes z+1 and z+2 still
+// add to.  Open nodes all have a = c = 1 and one b, so that a class id is only
+// looked up for its kind.  Order and rounding are those of k_update_iwb, in packed
+// pairs with uncontractible products.
+//
+// Measured on 512 x 384 x 256 FP32: 105 us of a 141 us step against 114 of 149 for
+// k_update_tma; HBM alone would take 96.  The shared-memory loads (12 wavefronts a
+// node and warp) bound it.  Two splits with fewer loads were slower: rows of 4 to
+// 8 nodes a thread from whole rows (117 against 90 us a step on 384 x 320 x 256, more
+// address arithmetic than loads saved), and 256 x 8 strips by one copy a row (160
+// us, the 26 copies of a plane).
+enum Kind : uint8_t { kOpen = 0, kOutside = 1, kClosure = 2 };
+
+__device__ __forceinline__ unsigned kind_of(uint32_t pos) {
+  return ((pos >> 30) & 1u) ? kClosure : (pos & 0x7Fu) == 0 ? kOutside : kOpen;
+}
+
+template <typename S, typename C>
+__global__ void __launch_bounds__(kThreads, 2)
+k_iwb_flat(const S* __restrict__ P, S* __restrict__ Pp, const S* __restrict__ past,
+           const C* __restrict__ cls, const uint32_t* __restrict__ pos, int n_classes, float b, int X,
+           int64_t XY, int z_last, int zc, int stages, float l2, float nzf, uint64_t wait_ns,
+           int* __restrict__ err) {
+  using namespace px;
+  using St = Store<S>;
+  constexpr bool kSmemTab = sizeof(C) == 1;
+  constexpr int kPairs = kPer / 2;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+  __shared__ uint8_t kinds[kSmemTab ? 256 : 1];
+  __shared__ __align__(8) uint64_t bars[2 * kMaxStages];
+  __shared__ int abort_flag;
+  const int halo = X + 1;
+  const Stage lay = stage_of(halo, sizeof(S), sizeof(C), 0);
+  const int t = threadIdx.x, lane = t & 31;
+  const int64_t s0 = (int64_t)blockIdx.x * kRange;
+  const int n = (int)(XY - s0 < kRange ? XY - s0 : (int64_t)kRange);
+  const int z0 = 1 + blockIdx.y * zc, z1 = min(z0 + zc, z_last), nplanes = z1 - z0;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * kMaxStages;
+  if (t == 0) {
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(full + 8 * i, 1);
+      mbar_init(empty + 8 * i, kConsumers / 32);
+    }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (kSmemTab)
+    for (int i = t; i < n_classes; i += kThreads) kinds[i] = (uint8_t)kind_of(pos[i]);
+  __syncthreads();
+  step_wait();
+  step_ready();
+  if (*(volatile int*)err) return;
+  if (nplanes <= 0) return;
+  if (t >= kConsumers) {
+    if (lane == 0)
+      produce<S, C>(smem, lay, full, empty, &abort_flag, P, past, cls, halo, XY, s0, n, z0, nplanes + 2,
+                    stages, 1, 0, err, wait_ns);
+    return;
+  }
+  const f2 nz = pk2(nzf, nzf), l22 = pk2(l2, l2), w1 = pk2(0.25f, 0.25f), w2 = pk2(0.125f, 0.125f),
+           w3 = pk2(0.0625f, 0.0625f), bb = pk2(b, b);
+  // The in-plane sums of stage k, handed pair by pair to `use`.
+  auto sums = [&](int k, auto&& use) {
+    const int64_t fp = (int64_t)(z0 - 1 + k) * XY + s0 - halo;
+    const S* p = (const S*)(smem + (size_t)(k % stages) * lay.bytes) + remainder_of<S>(fp) + halo + t;
+    const S *u = p - X, *d = p + X;
+#pragma unroll
+    for (int h = 0; h < kPairs; ++h) {
+      constexpr int o = kConsumers;
+      auto at = [&](const S* q, int x) { return pk2(St::load(q[2 * h * o + x]), St::load(q[2 * h * o + o + x])); };
+      use(h, at(p, 0), add2(add2(add2(at(u, 0), at(p, -1)), at(p, 1)), at(d, 0)),
+          add2(add2(add2(at(u, -1), at(u, 1)), at(d, -1)), at(d, 1)));
+    }
+  };
+  // of plane z: c0, c1, c2; of planes z and z-1 together: t1, t2, t3
+  f2 c0[kPairs], c1[kPairs], c2[kPairs], t1[kPairs], t2[kPairs], t3[kPairs];
+  bool ok = mbar_wait(full, 0, wait_ns) && mbar_wait(full + 8, 0, wait_ns);
+  if (ok) {
+    sums(0, [&](int h, f2 n0, f2 n1, f2 n2) { t1[h] = n0; t2[h] = n1; t3[h] = n2; });
+    sums(1, [&](int h, f2 n0, f2 n1, f2 n2) {
+      t1[h] = add2(n1, t1[h]);
+      t2[h] = add2(n2, t2[h]);
+      c0[h] = n0; c1[h] = n1; c2[h] = n2;
+    });
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(empty);
+      mbar_arrive(empty + 8);
+    }
+  }
+  for (int j = 0; j < nplanes && ok; ++j) {
+    const int sp = (j + 2) % stages;
+    ok = mbar_wait(full + 8 * sp, (uint32_t)(((j + 2) / stages) & 1), wait_ns);
+    if (!ok) break;
+    const int64_t fq = (int64_t)(z0 + j) * XY + s0;
+    const unsigned char* st = smem + (size_t)sp * lay.bytes;
+    const S* pq = (const S*)(st + lay.past) + remainder_of<S>(fq) + t;
+    const C* cl = (const C*)(st + lay.cls) + remainder_of<C>(fq) + t;
+    S* out = Pp + fq + t;
+    sums(j + 2, [&](int h, f2 n0, f2 n1, f2 n2) {
+      const int e0 = 2 * h * kConsumers, e1 = e0 + kConsumers;
+      const bool in0 = t + e0 < n, in1 = t + e1 < n;
+      const S v0 = pq[e0], v1 = pq[e1];
+      unsigned k0, k1;
+      if (kSmemTab) {
+        k0 = kinds[cl[e0]];
+        k1 = kinds[cl[e1]];
+      } else {
+        k0 = in0 ? kind_of(__ldg(pos + cl[e0])) : (unsigned)kOutside;
+        k1 = in1 ? kind_of(__ldg(pos + cl[e1])) : (unsigned)kOutside;
+      }
+      const f2 s1 = add2(t1[h], n0), s2 = add2(t2[h], n1), s3 = add2(t3[h], n2);
+      const f2 sw = fma2(l22, add2(add2(fma2(s1, w1, nz), fma2(s2, w2, nz)), fma2(s3, w3, nz)), nz);
+      const f2 o = sub2(add2(sw, fma2(bb, c0[h], nz)), pk2(St::load(v0), St::load(v1)));
+      float o0, o1;
+      up2(o, o0, o1);
+      const S r0 = k0 == kClosure ? v0 : St::store(k0 == kOutside ? 0.f : o0);
+      const S r1 = k1 == kClosure ? v1 : St::store(k1 == kOutside ? 0.f : o1);
+      if (in0) out[e0] = r0;
+      if (in1) out[e1] = r1;
+      t1[h] = add2(n1, c0[h]);
+      t2[h] = add2(n2, c1[h]);
+      t3[h] = c2[h];
+      c0[h] = n0; c1[h] = n1; c2[h] = n2;
+    });
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + 8 * sp);
+  }
+  if (!ok) {
+    atomicExch(err, 1);
+    *(volatile int*)&abort_flag = 1;
+  }
+}
+
 int flat_stages(const pfdtd_domain* d) {
-  const Stage lay = stage_of((int)(d->X * d->K), (int)d->esize, d->cls_bytes, d->kshift);
+  const int halo = (int)(d->X * d->K) + (d->class_scheme == PFDTD_IWB ? 1 : 0);
+  const Stage lay = stage_of(halo, (int)d->esize, d->cls_bytes, d->kshift);
   return (int)std::min<int64_t>(kMaxStages, (int64_t)((kSmemPerCta - 8192) / lay.bytes));
 }
 
-template <typename S, typename C, int SCHEME>
-int launch_flat_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
-  static std::atomic<bool> attr_done[64];
-  static std::mutex attr_mu;
-  if (d->device >= 64) return fail(PFDTD_ERR_UNSUPPORTED, "device index above 63");
-  if (!attr_done[d->device].load(std::memory_order_acquire)) {
-    std::lock_guard<std::mutex> lock(attr_mu);
-    PFDTD_CK(cudaFuncSetAttribute(k_update_flat<S, C, SCHEME>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+// The shared-memory opt-in of a kernel, once per device.
+template <typename K> int allow_smem(K kernel, std::atomic<bool>* done, std::mutex* mu, int device) {
+  if (device >= 64) return fail(PFDTD_ERR_UNSUPPORTED, "device index above 63");
+  if (!done[device].load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lock(*mu);
+    PFDTD_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kSmemPerCta - 6144)));
-    attr_done[d->device].store(true, std::memory_order_release);
+    done[device].store(true, std::memory_order_release);
   }
-  const int64_t nz = d->Z - 2, XYE = d->XY * d->K;
-  if (nz <= 0) return PFDTD_OK;
-  const int XE = (int)(d->X * d->K), stages = flat_stages(d);
-  const Stage lay = stage_of(XE, sizeof(S), sizeof(C), d->kshift);
-  const int64_t gx = (XYE + kRange - 1) / kRange;
-  // z-chunks as in launch_tma_t: two CTAs on an SM, four planes' cost a chunk
+  return PFDTD_OK;
+}
+
+// Planes per CTA, as in launch_tma_t: two CTAs on an SM, and a chunk
+// costs four planes more.
+int64_t flat_chunk(const pfdtd_domain* d, int64_t gx) {
+  const int64_t nz = d->Z - 2;
   int64_t best_c = 1;
   double best = 1e30;
   for (int64_t c = 1; c <= std::max<int64_t>(1, nz / 4); ++c) {
@@ -284,22 +438,58 @@ int launch_flat_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) 
     const double cost = (double)(waves * resident) / (double)ctas * (1.0 + 4.0 * (double)c / (double)nz);
     if (cost < best - 1e-9) { best = cost; best_c = c; }
   }
-  const int64_t zc = (nz + best_c - 1) / best_c;
+  return (nz + best_c - 1) / best_c;
+}
+
+ClassTab<float> class_table(const pfdtd_domain* d) {
   const char* tb = (const char*)d->d_ctab;
   const size_t n = d->n_classes;
-  ClassTab<float> tab{(const float*)tb, (const float*)(tb + 4 * n), (const float*)(tb + 8 * n),
-                      (const uint32_t*)(tb + 12 * n), d->n_classes};
+  return ClassTab<float>{(const float*)tb, (const float*)(tb + 4 * n), (const float*)(tb + 8 * n),
+                         (const uint32_t*)(tb + 12 * n), d->n_classes};
+}
+
+template <typename S, typename C, int SCHEME>
+int launch_flat_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
+  static std::atomic<bool> done[64];
+  static std::mutex mu;
+  const int64_t nz = d->Z - 2, XYE = d->XY * d->K;
+  if (nz <= 0) return PFDTD_OK;
+  if (int rc = allow_smem(k_update_flat<S, C, SCHEME>, done, &mu, d->device)) return rc;
+  const int XE = (int)(d->X * d->K), stages = flat_stages(d);
+  const int64_t gx = (XYE + kRange - 1) / kRange, zc = flat_chunk(d, gx);
+  const Stage lay = stage_of(XE, sizeof(S), sizeof(C), d->kshift);
   PFDTD_CK(launch_step_kernel(k_update_flat<S, C, SCHEME>, dim3((unsigned)gx, (unsigned)((nz + zc - 1) / zc)),
                               dim3(kThreads), (size_t)stages * lay.bytes + 128, s, (const S*)cur, (S*)past,
-                              (const S*)past, (const C*)d->d_cls, tab, XE, XYE, (int)(d->Z - 1), (int)zc,
-                              stages, d->K, d->kshift, (float)d->params[1], -0.0f, (unsigned)d->air_class,
-                              d->wait_ns, d->d_err));
+                              (const S*)past, (const C*)d->d_cls, class_table(d), XE, XYE,
+                              (int)(d->Z - 1), (int)zc, stages, d->K, d->kshift, (float)d->params[1],
+                              -0.0f, (unsigned)d->air_class, d->wait_ns, d->d_err));
   count_launch();
   return PFDTD_OK;
 }
 
 template <typename S, typename C>
+int launch_iwb_flat_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
+  static std::atomic<bool> done[64];
+  static std::mutex mu;
+  const int64_t nz = d->Z - 2;
+  if (nz > 0) {
+    if (int rc = allow_smem(k_iwb_flat<S, C>, done, &mu, d->device)) return rc;
+    const int stages = flat_stages(d);
+    const int64_t gx = (d->XY + kRange - 1) / kRange, zc = flat_chunk(d, gx);
+    const Stage lay = stage_of((int)d->X + 1, sizeof(S), sizeof(C), 0);
+    PFDTD_CK(launch_step_kernel(k_iwb_flat<S, C>, dim3((unsigned)gx, (unsigned)((nz + zc - 1) / zc)),
+                                dim3(kThreads), (size_t)stages * lay.bytes + 128, s, (const S*)cur,
+                                (S*)past, (const S*)past, (const C*)d->d_cls, class_table(d).pos,
+                                d->n_classes, d->iwb_open_b, (int)d->X, d->XY, (int)(d->Z - 1), (int)zc,
+                                stages, (float)d->params[1], -0.0f, d->wait_ns, d->d_err));
+    count_launch();
+  }
+  return launch_iwb_closure(d, cur, past, s);
+}
+
+template <typename S, typename C>
 int launch_flat_c(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
+  if (d->class_scheme == PFDTD_IWB) return launch_iwb_flat_t<S, C>(d, cur, past, s);
   if (d->class_scheme == PFDTD_SRL) return launch_flat_t<S, C, 1>(d, cur, past, s);
   if constexpr (std::is_same<S, float>::value) {
     if (d->class_form == PFDTD_FORM_DIFFERENCE) return launch_flat_t<S, C, 4>(d, cur, past, s);
@@ -315,12 +505,26 @@ int launch_flat_s(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) 
 
 }  // namespace
 
-// Whether the update of flat runs takes the rooms that k_update_tma does not:
-// 32-bit arithmetic, 7-point schemes, rows short enough for four stages.
+// Whether the update by flat runs can take the room: 32-bit arithmetic, rows
+// short enough for four stages; IWB with one field per node and its closure
+// list.
 bool flat_usable(const pfdtd_domain* d) {
-  return d->kernel_variant != PFDTD_KERNEL_ZMARCH && d->precision != PFDTD_F64 &&
-         d->class_scheme != PFDTD_IWB && d->X * d->K <= 4096 && d->XY * d->K < ((int64_t)1 << 31) &&
-         flat_stages(d) >= 4;
+  if (d->kernel_variant == PFDTD_KERNEL_ZMARCH || d->precision == PFDTD_F64) return false;
+  if (d->class_scheme == PFDTD_IWB && !(d->K == 1 && d->iwb_closure_ready && d->iwb_open)) return false;
+  return d->X * d->K <= 4096 && d->XY * d->K < ((int64_t)1 << 31) && flat_stages(d) >= 4;
+}
+
+// Whether the next IWB update is by flat runs with the closure pass.
+// Measured with DIF walls, us a step.  Rows that are not aligned, z-march / runs,
+// FP32: 203 x 155 x 119 33.7 / 21.6, 401 x 301 x 201 235 / 75.9, 131 x 127 x 125 24.0 /
+// 17.6; from about a million nodes (97 x 81 x 65 13.3 / 15.2), below which the closure pass costs more than the update saves.  Aligned rows, tiles /
+// runs, FP32: 160^3 30.2 / 24.4, 384 x 320 x 256 106.6 / 95.0, 512 x 384 x 256
+// 149.4 / 141.1, but 128^3 17.9 / 19.1; in FP16 512 x 384 x 256 150.6 / 157.2.
+bool iwb_flat(const pfdtd_domain* d) {
+  if (d->class_scheme != PFDTD_IWB || !flat_usable(d)) return false;
+  if (!uses_tma(d)) return d->kernel_variant == PFDTD_KERNEL_TMA || d->N >= 1000000;
+  return d->kernel_variant == PFDTD_KERNEL_AUTO && d->tma_tile < 0 && d->precision == PFDTD_F32 &&
+         d->N >= 3000000;
 }
 
 int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {

@@ -1191,7 +1191,8 @@ int launch_iwb_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s)
 bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
   // tile shapes 0..5 run the closure inside the streaming kernel
   return d->class_scheme == PFDTD_IWB && d->n_dif > 0 && d->iwb_closure_ready &&
-         d->d_iwb_closure_dif != nullptr && uses_tma(d) && !(d->tma_tile >= 0 && d->tma_tile <= 5);
+         d->d_iwb_closure_dif != nullptr &&
+         (iwb_flat(d) || (uses_tma(d) && !(d->tma_tile >= 0 && d->tma_tile <= 5)));
 }
 
 // Whether a room that the tiled kernel takes runs faster by flat runs
@@ -1204,7 +1205,7 @@ bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
 // 384 x 320 x 256 41.0 / 56.9).
 bool prefers_flat(const pfdtd_domain* d) {
   if (d->kernel_variant != PFDTD_KERNEL_AUTO || d->tma_tile >= 0 || d->K != 1) return false;
-  if (d->N < 3000000 || !flat_usable(d)) return false;
+  if (d->class_scheme == PFDTD_IWB || d->N < 3000000 || !flat_usable(d)) return false;
   if (d->precision != PFDTD_F32) return auto_tile16(d) == 0;
   return auto_tile(d) != 6 || (d->class_scheme != PFDTD_SRL && d->N >= 8000000);
 }

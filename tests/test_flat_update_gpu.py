@@ -114,9 +114,10 @@ def test_expired_wait_is_reported(gpu):
 
 
 @pytest.mark.parametrize("dims,scheme,prec", [((160, 140, 140), "forward", "f32"), ((160, 140, 140), "centred", "f32"),
-                                              ((160, 140, 140), "forward", "f16"), ((256, 200, 160), "forward", "f32")])
+                                              ((160, 140, 140), "forward", "f16"), ((256, 200, 160), "forward", "f32"),
+                                              ((160, 140, 140), "iwb", "f32"), ((109, 101, 97), "iwb", "f32")])
 def test_large_aligned_rooms(gpu, dims, scheme, prec):
-    """Rooms that the dispatch takes from the tiles equal the z-march kernel."""
+    """Rooms that the dispatch gives to the runs equal the z-march kernel."""
     room = rooms.boxes_room(dims, n_boxes=6, edge=(8, 40), n_materials=5, seed=3)
     P0 = _values(np.random.default_rng(1), room.n_nodes, prec)
     out = []
@@ -124,10 +125,57 @@ def test_large_aligned_rooms(gpu, dims, scheme, prec):
         with Domain(dims, prec) as d:
             d.set_kernel(kernel)
             d.set_scheme(scheme)
-            d.set_voxels(room.bid, room.mat, centred=scheme == "centred")
+            d.set_voxels(room.bid, room.mat, centred=scheme != "forward")
             d.set_materials(room.admittance)
-            d.set_params()
+            d.set_params(default_params(scheme="iwb" if scheme == "iwb" else "forward"))
             d.upload_field(L.FIELD_CURRENT, P0)
             d.run(5)
             out.append((d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("prec", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("dims,wide", [((5, 4, 5), False), ((45, 46, 12), False), ((683, 3, 6), False),
+                                       ((37, 29, 18), True), ((64, 33, 20), False), ((203, 31, 12), True),
+                                       ((100, 41, 24), True)])
+def test_iwb(gpu, O, prec, dims, wide):
+    """IWB by runs with the closure pass, inside nodes on the x and y faces,
+    frequency-dependent walls in half of the materials; rows with and without
+    16-byte alignment."""
+    from parallelfdtd_gb300 import materials
+    room = rooms.boxes_room(dims, n_boxes=2 if min(dims) > 16 else 0, edge=(4, 9), n_materials=6,
+                            seed=sum(dims))
+    X, Y, Z = dims
+    rng = np.random.default_rng(X)
+    bid, mat, table = room.bid.copy().reshape(Z, Y, X), room.mat.copy(), room.admittance
+    bid[2:-2, :, [0, -1]] = 26
+    bid[2:-2, [0, -1], :] = 26
+    bid = bid.reshape(-1)
+    if wide:
+        table = rooms.admittance_table(100, 0.05, 0.9, 9)
+        mat = np.where(bid > 0, rng.integers(0, 100, bid.size), 0).astype(np.uint8)
+    flags = np.array([m % 2 for m in range(len(table))], np.int32)
+    filters = materials.dif_table(materials.positive_real_filters(len(table), 3, seed=2), 3)
+    inside, steps = np.flatnonzero(bid), 7
+    src, rec = rng.choice(inside, 2), rng.choice(inside, 3)
+    pulses = rng.uniform(-1.0, 1.0, (2, steps))
+    P0, Pp0 = _values(rng, room.n_nodes, prec), _values(rng, room.n_nodes, prec)
+    params = default_params(scheme="iwb")
+    with Domain(dims, prec) as d:
+        d.set_kernel("tma")
+        d.set_scheme("iwb")
+        d.set_voxels(bid, mat, centred=True)
+        d.set_materials(table)
+        d.set_params(params)
+        d.set_dif_filters(flags, filters)
+        d.set_sources([room.coords(int(i)) for i in src], [1, 1], pulses)
+        d.set_receivers([room.coords(int(i)) for i in rec])
+        d.upload_field(L.FIELD_CURRENT, P0)
+        d.upload_field(L.FIELD_PAST, Pp0)
+        got, _, st = d.run(steps)
+        assert st == 0 and d.kernel() == "tma"
+        P, Pp = d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)
+    pos, m = O.encode_nodes(bid, mat, True)
+    want, rP, rPp = O.run(pos, m, dims, table, params, src, [1, 1], pulses, rec, steps, scheme=3,
+                          storage=None if prec == "f32" else prec, dif=(flags, filters), P0=P0, Pp0=Pp0)
+    assert np.array_equal(got, want) and np.array_equal(P, rP) and np.array_equal(Pp, rPp)
