@@ -494,7 +494,8 @@ def main():
     effective = bpu * nodes * K * T / (kms * 1e-3) / 1e9
     peak, peak_kind = peak_hbm()
     traffic = traffic_per_launch(prec, K, a.scheme)
-    kernel_name = "k_update_" + d.kernel()
+    # (the bulk-copy path takes tiles or flat runs by room size and alignment)
+    kernel_name = {"tma": "k_update_tma or k_update_flat"}.get(d.kernel(), "k_update_" + d.kernel())
     in_kernel_closure = os.environ.get("PFDTD_TMA_TILE", "-1").strip() in ("0", "1", "2", "3", "4", "5")
     if a.scheme == "iwb" and d.kernel() == "tma" and not in_kernel_closure:
         kernel_name += " + k_iwb_closure"  # the update of a step: both kernels, timed together

@@ -277,7 +277,7 @@ k_update_flat(const S* __restrict__ P, S* __restrict__ Pp, const S* __restrict__
 // looked up for its kind.  Order and rounding are those of k_update_iwb, in packed
 // pairs with uncontractible products.
 //
-// Measured on 512 x 384 x 256 FP32: 105 us of a 141 us step against 114 of 149 for
+// Measured on 512 x 384 x 256 FP32: 105 us of a 137 us step against 114 of 145 for
 // k_update_tma; HBM alone would take 96.  The shared-memory loads (12 wavefronts a
 // node and warp) bound it.  Two splits with fewer loads were slower: rows of 4 to
 // 8 nodes a thread from whole rows (117 against 90 us a step on 384 x 320 x 256, more
@@ -516,10 +516,12 @@ bool flat_usable(const pfdtd_domain* d) {
 
 // Whether the next IWB update is by flat runs with the closure pass.
 // Measured with DIF walls, us a step.  Rows that are not aligned, z-march / runs,
-// FP32: 203 x 155 x 119 33.7 / 21.6, 401 x 301 x 201 235 / 75.9, 131 x 127 x 125 24.0 /
-// 17.6; from about a million nodes (97 x 81 x 65 13.3 / 15.2), below which the closure pass costs more than the update saves.  Aligned rows, tiles /
-// runs, FP32: 160^3 30.2 / 24.4, 384 x 320 x 256 106.6 / 95.0, 512 x 384 x 256
-// 149.4 / 141.1, but 128^3 17.9 / 19.1; in FP16 512 x 384 x 256 150.6 / 157.2.
+// FP32: 203 x 155 x 119 33.6 / 19.6, 401 x 301 x 201 227 / 70.3, 131 x 127 x 125 24.0 /
+// 16.2; from about a million nodes (97 x 81 x 65 13.3 / 15.2), below which the
+// closure pass costs more than the update saves.  Aligned rows, tiles / runs, FP32:
+// 160^3 28.5 / 22.8, 384 x 320 x 256 103.9 / 91.6, 512 x 384 x 256 144.9 / 136.6,
+// 256 x 192 x 128 29.7 / 29.3, 128^3 no difference (without walls 17.0 / 18.2); in
+// FP16 512 x 384 x 256 without walls 150.6 / 157.2.
 bool iwb_flat(const pfdtd_domain* d) {
   if (d->class_scheme != PFDTD_IWB || !flat_usable(d)) return false;
   if (!uses_tma(d)) return d->kernel_variant == PFDTD_KERNEL_TMA || d->N >= 1000000;
