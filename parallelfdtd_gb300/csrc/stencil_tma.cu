@@ -924,9 +924,10 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // first stages arrive, about two planes' more (chunks of 16 planes or more
   // left small rooms to a few CTAs: 10 us an update on 48 x 40 x 36, 3.9
   // now).  FP64 is bound by its operations, which the loads do not add to
-  // (100 x 90 x 80, 8 fields: 195 -> 135 us).
+  // (100 x 90 x 80, 8 fields: 195 -> 135 us); 16-bit tiles, nearer to that, do
+  // with two planes (448 x 320 x 240 FP16 68.4 -> 63.4 us).
   constexpr int kMinPlanes = 4;
-  constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : 4.0;
+  constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : sizeof(S) == 2 ? 2.0 : 4.0;
   const int64_t per_sm =
       occ > 0
           ? occ
@@ -952,9 +953,9 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
   // Large 16-bit rooms are launched plainly: an update set up while the one
   // before drains streams 3 % slower there than its gap costs (512 x 384 x 256:
-  // 65.1 us a step, 61.1 plainly; 512 x 384 x 200 centred BF16 74.8, 73.5), while
+  // 65.1 us a step, 61.1 plainly; 512 x 384 x 200 centred BF16 74.8, 72.1), while
   // 384 x 320 x 256 takes 43.0 against 45.5.
-  const bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 35000000);
+  const bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000);
   PFDTD_CK(launch_kernel(
       dependent, k_update_tma<S, C, SCHEME, Lay, BATCHED>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
       ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur, (S*)past,
@@ -1205,13 +1206,13 @@ bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
 // (256^3 36.9 / 34.0, 512 x 384 x 256 99.9 / 95.8; 240 x 200 x 160 15.6 / 16.3), and
 // from 3 M where 256-wide tiles do not cover the rows (160^3 11.2 / 9.7, 320 x 240 x
 // 200 38.1 / 30.5, 128 x 150 x 150 of 2.9 M 7.6 / 7.8); centred only the latter
-// (384 x 320 x 256 74.7 / 71.2, 512 x 384 x 256 106 / 110); 16-bit fields, whose
-// tiles carry 8 nodes a thread, where only 64-wide tiles fit (160^3 11.9 / 10.4,
-// 384 x 320 x 256 41.0 / 56.9).
+// (384 x 320 x 256 74.7 / 71.2, 512 x 384 x 256 106 / 110); 16-bit fields
+// where only 64-wide tiles fit, to 5 M nodes (a step of 160^3 FP16 13.7 / 12.2, centred
+// 15.7 / 15.4; 176^3 15.6 / 15.4, centred 18.2 / 20.4; 320 x 200 x 160 22.5 / 24.0).
 bool prefers_flat(const pfdtd_domain* d) {
   if (d->kernel_variant != PFDTD_KERNEL_AUTO || d->tma_tile >= 0 || d->K != 1) return false;
   if (d->class_scheme == PFDTD_IWB || d->N < 3000000 || !flat_usable(d)) return false;
-  if (d->precision != PFDTD_F32) return auto_tile16(d) == 0;
+  if (d->precision != PFDTD_F32) return auto_tile16(d) == 0 && d->N < 5000000;
   return auto_tile(d) != 6 || (d->class_scheme != PFDTD_SRL && d->N >= 8000000);
 }
 
