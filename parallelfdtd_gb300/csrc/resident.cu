@@ -249,7 +249,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
   __shared__ int l_src[kMaxSources], l_rec[kMaxReceivers];   // shared-memory offsets
   __shared__ int l_src_id[kMaxSources], l_rec_id[kMaxReceivers];
   __shared__ int n_lsrc, n_lrec, gave_up;
-  if (*(volatile int*)g.err) return;
+  // One thread reads the flag, and the block leaves or stays as a whole: a block
+  // of this launch whose wait expires may raise it while this one starts, and a
+  // block that some threads have left would run on tables they never filled.
+  if (threadIdx.x == 0) n_lsrc = n_lrec = gave_up = 0;
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)g.err != 0)) return;
   const Brick& k = g.k;
   // Rows of the brick start 4 values into a row of the array.  The left halo
   // node lies in the value before; the right one after the row, which may be
@@ -337,7 +341,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
     if (lane == 0) {
       n_lsrc = ns;
       n_lrec = nr;
-      gave_up = 0;
     }
   }
 

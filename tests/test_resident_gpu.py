@@ -144,3 +144,33 @@ def test_other_rooms_take_the_general_path(gpu, O, place):
     want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(),
                         [room.flat(*place)], [1], pulse, [room.flat(24, 20, 18)], 40)
     assert np.array_equal(got, want) and np.array_equal(P, rP)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_expired_wait_is_reported(gpu, O, prec):
+    """A wait bound of a nanosecond runs out in the exchange of faces: the run
+    fails, with the context and the domain usable, and the next one, the bound
+    restored, equals the oracle (its step tags go on after those of the run
+    that broke off)."""
+    room, steps = rooms.shoebox((64, 60, 56), seed=1), 40
+    src, rec, pulse = (32, 30, 28), (20, 30, 40), rooms.gaussian_pulse(40, 3.0)[None]
+    with Domain(room.dims, prec) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([src], [1], pulse)
+        d.set_receivers([rec])
+        L.call("pfdtd_set_wait_limit", d.handle, 1)
+        for _ in range(3):
+            with pytest.raises(L.PfdtdError) as e:
+                d.run(2000)
+            assert e.value.status == L.ERR_CUDA and "timed out" in str(e.value)
+        L.call("pfdtd_set_wait_limit", d.handle, 0)
+        d.reset_fields()
+        got, _, st = d.run(steps)
+        assert st == 0
+        P = d.download_field(L.FIELD_CURRENT)
+    pos, mat = O.encode_nodes(room.bid, room.mat, False)
+    want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(), [room.flat(*src)], [1],
+                        pulse, [room.flat(*rec)], steps, double=prec == "f64")
+    assert np.abs(want).max() > 0 and np.array_equal(got, want) and np.array_equal(P, rP)
