@@ -221,6 +221,12 @@ int prepare_run(pfdtd_domain* d) {
   return PFDTD_OK;
 }
 
+// Whether a resident launch was refused (not failed): the first launch of a
+// run is, if any, so that the whole run takes single steps.
+bool resident_refused(const pfdtd_domain* d, int rc) {
+  return rc == PFDTD_ERR_UNSUPPORTED && !d->resident.ok;
+}
+
 // Steps of one resident launch when nobody asks between chunks.
 constexpr int64_t kResidentChunk = 8192;
 
@@ -266,8 +272,10 @@ int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool
                 int64_t* steps_queued, bool poll = true, int64_t resident_chunk = kResidentChunk) {
   // (asynchronous runs share the GPU with other domains' runs and keep to
   // single steps: a resident launch would hold every SM for its whole length)
-  if (poll && resident_usable(d))
-    return enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, resident_chunk);
+  if (poll && resident_usable(d)) {
+    const int rc = enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, resident_chunk);
+    if (!resident_refused(d, rc) || *steps_queued > 0) return rc;
+  }
   cudaStream_t s = d->stream;
   PFDTD_CK(cudaMemsetAsync(d->d_step, 0, sizeof(int64_t), s));
   if (int rc0 = launch_dif_init(d, s)) return rc0;
@@ -328,11 +336,10 @@ int enqueue_steps(pfdtd_domain* d, int64_t at, int64_t n, void* rec_out, int64_t
                   int64_t inject_end) {
   cudaStream_t s = d->stream;
   if (resident_usable(d)) {
-    for (int64_t done = 0; done < n; done += kResidentChunk)
-      if (int rc = launch_resident(d, at + done, std::min(kResidentChunk, n - done), rec_out, rec_ld,
-                                   inject_end, s))
-        return rc;
-    return PFDTD_OK;
+    int rc = PFDTD_OK;
+    for (int64_t i = 0; i < n && rc == PFDTD_OK; i += kResidentChunk)
+      rc = launch_resident(d, at + i, std::min(kResidentChunk, n - i), rec_out, rec_ld, inject_end, s);
+    if (!resident_refused(d, rc) || at > 0) return rc;
   }
   const int tb = tb_active(d) ? d->tb_depth : 0;
   const int64_t chunk = tb ? kChunkTb : kChunk;

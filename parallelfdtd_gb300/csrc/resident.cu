@@ -666,9 +666,19 @@ int launch_nz(pfdtd_domain* d, const Args<S>& a, cudaStream_t s) {
     attr_done[d->device].store(true, std::memory_order_release);
   }
   void* args[] = {(void*)&a};
-  PFDTD_CK(cudaLaunchCooperativeKernel((const void*)k_resident<S, SCHEME, NZ>,
-                                       dim3(a.k.gx * a.k.gy * a.k.gz), dim3(kThreads), args,
-                                       brick_smem<A>(a.k), s));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void*)k_resident<S, SCHEME, NZ>,
+                                  dim3(a.k.gx * a.k.gy * a.k.gz), dim3(kThreads), args,
+                                  brick_smem<A>(a.k), s);
+  // Refused as a whole, where the process may not use as many SMs at once as
+  // there are bricks: nothing has run, and the domain keeps to single steps.
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+      e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    d->resident.ok = false;
+    return PFDTD_ERR_UNSUPPORTED;
+  }
+  PFDTD_CK(e);
   count_launch();
   return PFDTD_OK;
 }
@@ -739,8 +749,8 @@ int launch_t(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64
 }  // namespace
 
 // Whether the domain's steps can run resident; plans the bricks and allocates
-// the inboxes on the first call for a class build (a failed allocation leaves
-// the per-step path in use).
+// the inboxes on the domain's first call (a failed allocation or a refused
+// launch leaves the per-step path in use).
 bool resident_usable(pfdtd_domain* d) {
   if (d->kernel_variant != PFDTD_KERNEL_AUTO || d->tma_tile >= 0 || d->tb_depth >= 2) return false;
   if (d->K != 1 || d->Z < 3 || !d->tb_faces_ok || d->n_dif > 0) return false;
@@ -780,6 +790,7 @@ bool resident_usable(pfdtd_domain* d) {
 
 // Queue steps [step0, step0 + steps) as one launch: sources injected,
 // receivers recorded, fields and their roles as after that many single steps.
+// PFDTD_ERR_UNSUPPORTED with resident.ok cleared: refused, nothing queued.
 int launch_resident(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64_t rec_ld,
                     int64_t inject_end, cudaStream_t s) {
   ResidentState& rs = d->resident;

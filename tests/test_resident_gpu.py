@@ -5,6 +5,10 @@ each axis, one brick, one node of air, long and flat rooms, and the largest
 number of planes a thread holds.  Fields start from random values, planes 0 and
 Z-1 (never updated) included, and the step counts are odd, so that both buffers
 of a halo exchange and both field roles are used."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -174,3 +178,52 @@ def test_expired_wait_is_reported(gpu, O, prec):
     want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(), [room.flat(*src)], [1],
                         pulse, [room.flat(*rec)], steps, double=prec == "f64")
     assert np.abs(want).max() > 0 and np.array_equal(got, want) and np.array_equal(P, rP)
+
+
+_REFUSED = """
+import sys
+import numpy as np
+from tests.test_resident_gpu import _refusal_run
+from parallelfdtd_gb300 import _lib
+before = _lib.load().pfdtd_kernel_launches()
+out = _refusal_run()
+np.savez(sys.argv[1], *out, launches=_lib.load().pfdtd_kernel_launches() - before)
+"""
+
+
+def _refusal_run():
+    room, steps = rooms.shoebox((48, 40, 36), seed=1), 70
+    with Domain(room.dims) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([(24, 20, 18)], [1], rooms.gaussian_pulse(steps, 3.0)[None])
+        d.set_receivers([(20, 10, 30)])
+        a = d.run(steps)[0]
+        P = d.download_field(L.FIELD_CURRENT)
+        d.reset_fields()
+        b, caps = d.run_captures(steps, [(0, 0, 18), (30, 1, 20), (70, 2, 24)])
+        d.reset_fields()
+        seen = []
+        c = d.run(steps, progress=lambda s, n, t: seen.append(s))[0]
+        assert seen == [0]
+    return [a, P, b, c] + [p for p, _ in caps]
+
+
+@pytest.mark.parametrize("code", [720, 701, 801])
+def test_refused_cooperative_launch(gpu, tmp_path, code):
+    """Where the runtime refuses a cooperative launch (a stand-in for the call
+    answers with its error codes: too large, out of resources, not supported),
+    runs take single steps and give the same results."""
+    src, lib, out = tmp_path / "refuse.cpp", tmp_path / "refuse.so", tmp_path / "out.npz"
+    src.write_text('extern "C" int cudaLaunchCooperativeKernel(...) { return %d; }\n' % code)
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, LD_PRELOAD=str(lib), PYTHONPATH=root)
+    r = subprocess.run([sys.executable, "-c", _REFUSED, str(out)], cwd=root, env=env, timeout=120,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    got = np.load(out)
+    assert got["launches"] > 3 * 2 * 70  # update and step I/O of every step
+    for i, v in enumerate(_refusal_run()):
+        assert np.array_equal(got["arr_%d" % i], v), i
