@@ -272,6 +272,7 @@ struct ResidentState {
   int words = 0;             // of one brick's inbox half
   size_t bytes = 0;
   uint32_t tag = 1;          // of the next step
+  int64_t chunk = 0;         // steps of one launch
 };
 
 }  // namespace pfdtd

@@ -227,9 +227,6 @@ bool resident_refused(const pfdtd_domain* d, int rc) {
   return rc == PFDTD_ERR_UNSUPPORTED && !d->resident.ok;
 }
 
-// Steps of one resident launch when nobody asks between chunks.
-constexpr int64_t kResidentChunk = 8192;
-
 // enqueue_run for a grid that stays on the SMs (resident.cu): launches of
 // `chunk` steps instead of graphs of single steps.
 template <typename F>
@@ -269,11 +266,12 @@ int enqueue_resident(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between,
 // completion; it returns non-zero to stop.
 template <typename F>
 int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool* stopped,
-                int64_t* steps_queued, bool poll = true, int64_t resident_chunk = kResidentChunk) {
-  // (asynchronous runs share the GPU with other domains' runs and keep to
-  // single steps: a resident launch would hold every SM for its whole length)
+                int64_t* steps_queued, bool poll = true, bool asked = false) {
+  // (asynchronous runs are many at a time and keep to single steps, which
+  // share the SMs; a resident launch holds them all)
   if (poll && resident_usable(d)) {
-    const int rc = enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, resident_chunk);
+    const int64_t chunk = asked ? std::min(kChunk, d->resident.chunk) : d->resident.chunk;
+    const int rc = enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, chunk);
     if (!resident_refused(d, rc) || *steps_queued > 0) return rc;
   }
   cudaStream_t s = d->stream;
@@ -336,9 +334,10 @@ int enqueue_steps(pfdtd_domain* d, int64_t at, int64_t n, void* rec_out, int64_t
                   int64_t inject_end) {
   cudaStream_t s = d->stream;
   if (resident_usable(d)) {
+    const int64_t chunk = d->resident.chunk;
     int rc = PFDTD_OK;
-    for (int64_t i = 0; i < n && rc == PFDTD_OK; i += kResidentChunk)
-      rc = launch_resident(d, at + i, std::min(kResidentChunk, n - i), rec_out, rec_ld, inject_end, s);
+    for (int64_t i = 0; i < n && rc == PFDTD_OK; i += chunk)
+      rc = launch_resident(d, at + i, std::min(chunk, n - i), rec_out, rec_ld, inject_end, s);
     if (!resident_refused(d, rc) || at > 0) return rc;
   }
   const int tb = tb_active(d) ? d->tb_depth : 0;
@@ -738,7 +737,7 @@ int pfdtd_run(pfdtd_domain* d, int64_t steps, void* out, pfdtd_interrupt_fn inte
   bool stopped = false;
   int64_t queued = 0;
   rc = enqueue_run(d, steps, d->d_rec_out, between, &stopped, &queued, true,
-                   interrupt_cb || progress_cb ? kChunk : kResidentChunk);
+                   interrupt_cb || progress_cb);
   if (rc) return rc;
   // Rows of receivers outside the grid are left untouched (kernels3d.cu:184-191).
   const size_t row = (size_t)steps * d->arith_size();

@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
 // memory bandwidth), its face nodes (a third of a cycle each) and a fixed
 // exchange latency.  false: the grid does not fit.
 template <typename A>
-bool plan_bricks(const pfdtd_domain* d, int max_planes, Brick* out) {
+bool plan_bricks(const pfdtd_domain* d, int max_planes, Brick* out, double* cycles) {
   double best = 1e30;
   const int64_t nz = d->Z - 2;
   for (int gx = 1; gx <= d->sm_count && gx <= d->X; ++gx) {
@@ -650,6 +650,7 @@ bool plan_bricks(const pfdtd_domain* d, int max_planes, Brick* out) {
       }
     }
   }
+  *cycles = best;
   return best < 1e30;
 }
 
@@ -746,6 +747,14 @@ int launch_t(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64
   return launch_scheme<S, 0>(d, a, s);
 }
 
+// A resident launch holds every SM until it ends, and work of other streams
+// waits behind it.  About a millisecond of it at a time is no more than they wait
+// behind one update of a large batch (0.9 ms).  With 8192 steps a launch a single
+// step beside a 64^3 run in another thread waited 21 ms, now 0.7 (at most 2);
+// long runs take 1 % longer so at 64^3, 3 % at 128^3 (2 ms: 0.6, at most 4; 0.5 ms:
+// 0.3, at most 1, but 2 % and 6 %).
+constexpr double kLaunchNs = 1e6;
+
 }  // namespace
 
 // Whether the domain's steps can run resident; plans the bricks and allocates
@@ -767,9 +776,12 @@ bool resident_usable(pfdtd_domain* d) {
     rs.planned = true;
     rs.ok = false;
     Brick k{};
-    const bool fits = d->precision == PFDTD_F64 ? plan_bricks<double>(d, kMaxPlanes, &k)
-                                                : plan_bricks<float>(d, kMaxPlanes, &k);
+    double cycles = 0.0;
+    const bool fits = d->precision == PFDTD_F64 ? plan_bricks<double>(d, kMaxPlanes, &k, &cycles)
+                                                : plan_bricks<float>(d, kMaxPlanes, &k, &cycles);
     if (!fits) return false;
+    const double step_ns = 0.7 * cycles + (d->precision == PFDTD_F64 ? 0.03 * (double)d->N : 0.0);
+    rs.chunk = std::max<int64_t>(2, (int64_t)(kLaunchNs / step_ns));
     const int words = inbox_values(k) * (int)(d->arith_size() / 4);
     const size_t bytes = 2 * sizeof(uint64_t) * (size_t)words * k.gx * k.gy * k.gz;
     if (d->alloc(&rs.inbox, bytes) != cudaSuccess) {

@@ -123,6 +123,29 @@ def test_chunks_with_progress(gpu, O):
     assert seen == [0, 100]
 
 
+def test_long_run_is_cut_into_launches(gpu, O):
+    """A run of 2500 steps holds the SMs for about a millisecond at a time: it is
+    several launches, and as the oracle has it."""
+    launches = L.load().pfdtd_kernel_launches
+    room, steps = rooms.shoebox((24, 24, 24), seed=2), 2500
+    src, rec, pulse = (12, 12, 12), (5, 6, 7), rooms.gaussian_pulse(2500, 3.0)[None]
+    with Domain(room.dims) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([src], [1], pulse)
+        d.set_receivers([rec])
+        d.run(50)
+        d.reset_fields()
+        before = launches()
+        got, _, st = d.run(steps)
+        assert st == 0 and 3 <= launches() - before <= 50
+    pos, mat = O.encode_nodes(room.bid, room.mat, False)
+    want, _, _ = O.run(pos, mat, room.dims, room.admittance, default_params(), [room.flat(*src)], [1],
+                       pulse, [room.flat(*rec)], steps)
+    assert np.array_equal(got, want)
+
+
 def test_captures(gpu, O):
     _check(O, (52, 36, 45), "f32", "forward", 31, captures=(0, 4, 5, 31))
 
