@@ -452,6 +452,7 @@ int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_
 bool prefers_flat(const pfdtd_domain* d);  // stencil_tma.cu
 // Implemented in resident.cu
 bool resident_usable(pfdtd_domain* d);
+bool resident_pays(pfdtd_domain* d, int64_t steps);
 int launch_resident(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out, int64_t rec_ld,
                     int64_t inject_end, cudaStream_t s);
 // Implemented in stencil_tb.cu

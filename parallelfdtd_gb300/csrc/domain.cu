@@ -269,7 +269,7 @@ int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool
                 int64_t* steps_queued, bool poll = true, bool asked = false) {
   // (asynchronous runs are many at a time and keep to single steps, which
   // share the SMs; a resident launch holds them all)
-  if (poll && resident_usable(d)) {
+  if (poll && resident_pays(d, steps)) {
     const int64_t chunk = asked ? std::min(kChunk, d->resident.chunk) : d->resident.chunk;
     const int rc = enqueue_resident(d, steps, rec_out, between, stopped, steps_queued, chunk);
     if (!resident_refused(d, rc) || *steps_queued > 0) return rc;
@@ -329,16 +329,18 @@ int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool
 // Queue `n` steps continuing from step `at` (also the device step counter),
 // without host waits: resident launches, or chunk graphs for whole chunks, then
 // blocked launches and single steps.  rec_ld / inject_end as in enqueue_run
-// (the run's step count).
+// (the run's step count).  `resident`: the same for the whole run; cleared when
+// the first launch is refused.
 int enqueue_steps(pfdtd_domain* d, int64_t at, int64_t n, void* rec_out, int64_t rec_ld,
-                  int64_t inject_end) {
+                  int64_t inject_end, bool* resident) {
   cudaStream_t s = d->stream;
-  if (resident_usable(d)) {
+  if (*resident) {
     const int64_t chunk = d->resident.chunk;
     int rc = PFDTD_OK;
     for (int64_t i = 0; i < n && rc == PFDTD_OK; i += chunk)
       rc = launch_resident(d, at + i, std::min(chunk, n - i), rec_out, rec_ld, inject_end, s);
     if (!resident_refused(d, rc) || at > 0) return rc;
+    *resident = false;
   }
   const int tb = tb_active(d) ? d->tb_depth : 0;
   const int64_t chunk = tb ? kChunkTb : kChunk;
@@ -821,10 +823,17 @@ int pfdtd_run_captures(pfdtd_domain* d, int64_t steps, void* out, int n_cap,
   uint8_t* sq = (uint8_t*)stage + (size_t)total * 4;
   PFDTD_CK(cudaMemsetAsync(d->d_step, 0, sizeof(int64_t), s));
   rc = launch_dif_init(d, s);
-  int64_t at = 0;
+  // pieces that the captures cut the run into
+  int64_t pieces = 1, at = 0;
+  for (int i : order) {
+    pieces += cap_step[i] > at && cap_step[i] < steps;
+    at = cap_step[i];
+  }
+  bool resident = resident_pays(d, steps / pieces);
+  at = 0;
   for (int k = 0; k < n_cap && rc == PFDTD_OK; ++k) {
     const int i = order[k];
-    rc = enqueue_steps(d, at, cap_step[i] - at, d->d_rec_out, steps, steps);
+    rc = enqueue_steps(d, at, cap_step[i] - at, d->d_rec_out, steps, steps, &resident);
     at = cap_step[i];
     if (rc) break;
     float* dp = p_out && p_out[i] ? sp + offset[i] : nullptr;
@@ -836,9 +845,9 @@ int pfdtd_run_captures(pfdtd_domain* d, int64_t steps, void* out, int n_cap,
     if (e == cudaSuccess && dq) e = cudaMemcpyAsync(pos_out[i], dq, size[i], cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) rc = cuda_fail(e, "capture copy", __FILE__, __LINE__);
   }
-  if (rc == PFDTD_OK) rc = enqueue_steps(d, at, steps - at, d->d_rec_out, steps, steps);
+  if (rc == PFDTD_OK) rc = enqueue_steps(d, at, steps - at, d->d_rec_out, steps, steps, &resident);
   // record the receivers of the last step (resident launches have); never inject
-  if (rc == PFDTD_OK && steps > 0 && !resident_usable(d)) rc = launch_io(d, d->cur_field(), d->d_rec_out, steps, 0, s);
+  if (rc == PFDTD_OK && steps > 0 && !resident) rc = launch_io(d, d->cur_field(), d->d_rec_out, steps, 0, s);
   if (rc == PFDTD_OK) {
     const size_t row = (size_t)steps * d->arith_size();
     for (int r = 0; r < d->n_rec && rc == PFDTD_OK && steps > 0; ++r)

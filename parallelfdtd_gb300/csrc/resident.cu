@@ -800,6 +800,15 @@ bool resident_usable(pfdtd_domain* d) {
   return rs.ok;
 }
 
+// Whether `steps` steps at a time run faster resident than one by one.  A launch
+// fills the SMs and empties them again, which costs two or three single steps and
+// more the more nodes there are.  Measured, us a call, resident / single steps:
+// 24^3 of 1 step 51 / 45, of 3 50 / 60; 64^3 of 1 51 / 46, of 4 55 / 66; 128^3 of 1 75 /
+// 55, of 8 113 / 105, of 12 131 / 134.
+bool resident_pays(pfdtd_domain* d, int64_t steps) {
+  return steps >= 3 + d->N / 230000 && resident_usable(d);
+}
+
 // Queue steps [step0, step0 + steps) as one launch: sources injected,
 // receivers recorded, fields and their roles as after that many single steps.
 // PFDTD_ERR_UNSUPPORTED with resident.ok cleared: refused, nothing queued.

@@ -146,6 +146,37 @@ def test_long_run_is_cut_into_launches(gpu, O):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("dims,steps,resident", [((24, 24, 24), 2, False), ((24, 24, 24), 3, True),
+                                                 ((128, 128, 128), 11, False), ((128, 128, 128), 12, True)])
+def test_short_runs_take_single_steps(gpu, O, dims, steps, resident):
+    """Filling and emptying the SMs costs some single steps' time: a run of fewer
+    takes those, also between captures, and gives the same results."""
+    launches = L.load().pfdtd_kernel_launches
+    room, src, rec = rooms.shoebox(dims, seed=2), (12, 12, 12), (11, 12, 13)
+    P0 = _values(np.random.default_rng(1), room.n_nodes, "f32")
+    pulse = rooms.gaussian_pulse(5 * steps, 3.0)[None]
+    caps = [(steps, 0, 12)] * 2 + [(2 * steps, 1, 12), (2 * steps, 2, 12)]  # three pieces
+    with Domain(dims) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([src], [1], pulse)
+        d.set_receivers([rec])
+        d.run(50)  # classes, plan
+        got = []
+        for run in (lambda: d.run(steps)[0], lambda: d.run_captures(3 * steps, caps)[0]):
+            d.reset_fields()
+            d.upload_field(L.FIELD_CURRENT, P0)
+            before = launches()
+            got.append((run(), launches() - before, d.download_field(L.FIELD_CURRENT)))
+    assert (got[0][1] == 1) == resident and (got[1][1] == 3 + len(caps)) == resident
+    pos, mat = O.encode_nodes(room.bid, room.mat, False)
+    for (r, _, P), n in zip(got, (steps, 3 * steps)):
+        want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(), [room.flat(*src)],
+                            [1], pulse[:, :n], [room.flat(*rec)], n, P0=P0)
+        assert np.array_equal(r, want) and np.array_equal(P, rP)
+
+
 def test_captures(gpu, O):
     _check(O, (52, 36, 45), "f32", "forward", 31, captures=(0, 4, 5, 31))
 
