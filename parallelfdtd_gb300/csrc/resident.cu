@@ -604,8 +604,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
 
 // The split of the grid into at most `sms` bricks with the least estimated
 // time a step: the busiest CTA's warp-planes (about 30 cycles each: shared
-// memory bandwidth), its face nodes (a third of a cycle each) and a fixed
-// exchange latency.  false: the grid does not fit.
+// memory bandwidth; in double about 900, its operations), its face nodes (a third
+// of a cycle each) and a fixed exchange latency.  (With 60 cycles for doubles a
+// 16^3 room was one brick: 15.2 us a step, 3.1 in many.)  false: the grid does not
+// fit.
 template <typename A>
 bool plan_bricks(const pfdtd_domain* d, int max_planes, Brick* out, double* cycles) {
   double best = 1e30;
@@ -641,8 +643,8 @@ bool plan_bricks(const pfdtd_domain* d, int max_planes, Brick* out, double* cycl
         const int warps = (ncol * k.groups + 31) / 32;
         const double faces = (k.gx > 1 ? 2.0 * k.by * k.bz : 0) + (k.gy > 1 ? 2.0 * k.bx * k.bz : 0) +
                              (k.gz > 1 ? 2.0 * k.bx * k.by : 0);
-        const double cost =
-            sizeof(A) / 4 * (30.0 * k.planes * warps + 0.35 * faces) + (faces > 0 ? 2500.0 : 500.0);
+        const double cost = (sizeof(A) == 8 ? 900.0 : 30.0) * k.planes * warps +
+                            0.35 * (sizeof(A) / 4) * faces + (faces > 0 ? 2500.0 : 500.0);
         if (cost < best) {
           best = cost;
           *out = k;
@@ -687,9 +689,18 @@ int launch_nz(pfdtd_domain* d, const Args<S>& a, cudaStream_t s) {
 // Register arrays are sized at compile time: the smallest that holds the
 // plan's planes per thread.  Eight planes of 4 nodes for 512 threads are 2.4 M
 // nodes on the whole chip.  With 12 and 17 planes the FP32 kernel spilled: it
-// took 13.2 us a step on 160^3 where single steps take 15.2, and 15.1 against
-// 14.7 on 203 x 155 x 119, so larger rooms keep to single steps.
+// took 13.2 us a step on 160^3 and 15.1 on 203 x 155 x 119, where single steps
+// take 10.8, so larger rooms keep to single steps.  At the line, us a step,
+// resident / single: FP32 forward 128^3 5.2 / 6.6, 128 x 150 x 124 6.5 / 7.2, 131 x 127
+// x 125 6.8 / 8.6, centred 6.3 / 7.1, 7.8 / 7.7 and 7.7 / 10.7; FP16 forward 5.3 / 6.3, 6.6 /
+// 6.4 and 7.0 / 9.0.
 constexpr int kMaxPlanes = 8;
+// Nodes per SM of an FP64 room.  The z-march kernel keeps the FP64 units busier
+// once it fills the SMs.  Forward and centred, us a step, resident / single: 64^3
+// 8.2 / 9.8 and 12.8 / 15.6, 96^3 26.1 / 22.2 and 40.6 / 60.8, 120 x 110 x 100 37.4 / 41.1
+// and 59.7 / 61.1; beyond the line 130 x 100 x 105 42.0 / 40.9 and 65.9 / 64.5, 128^3
+// 57.9 / 49.3 and 93.1 / 78.5.
+constexpr int kMostDoubles = 8700;
 
 template <typename S, int SCHEME>
 int launch_scheme(pfdtd_domain* d, const Args<S>& a, cudaStream_t s) {
@@ -766,7 +777,7 @@ bool resident_usable(pfdtd_domain* d) {
   if (d->class_scheme != PFDTD_SRL_FORWARD && d->class_scheme != PFDTD_SRL) return false;
   if (d->cls_bytes != 1 || d->n_classes > 255) return false;  // one id for nodes past the grid
   if (d->n_src > kMaxSources || d->n_rec > kMaxReceivers) return false;
-  if (d->N > (int64_t)d->sm_count * 40000) return false;
+  if (d->N > (int64_t)d->sm_count * (d->precision == PFDTD_F64 ? kMostDoubles : 40000)) return false;
   for (int64_t e : d->src_idx_h)
     if (e >= 0 && (e < d->XY || e >= d->N - d->XY)) return false;
   for (int64_t e : d->rec_idx_h)
@@ -780,8 +791,7 @@ bool resident_usable(pfdtd_domain* d) {
     const bool fits = d->precision == PFDTD_F64 ? plan_bricks<double>(d, kMaxPlanes, &k, &cycles)
                                                 : plan_bricks<float>(d, kMaxPlanes, &k, &cycles);
     if (!fits) return false;
-    const double step_ns = 0.7 * cycles + (d->precision == PFDTD_F64 ? 0.03 * (double)d->N : 0.0);
-    rs.chunk = std::max<int64_t>(2, (int64_t)(kLaunchNs / step_ns));
+    rs.chunk = std::max<int64_t>(2, (int64_t)(kLaunchNs / (0.7 * cycles)));
     const int words = inbox_values(k) * (int)(d->arith_size() / 4);
     const size_t bytes = 2 * sizeof(uint64_t) * (size_t)words * k.gx * k.gy * k.gz;
     if (d->alloc(&rs.inbox, bytes) != cudaSuccess) {

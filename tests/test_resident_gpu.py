@@ -112,6 +112,30 @@ def test_largest_double(gpu, O):
     _check(O, (128, 100, 98), "f64", "forward", 21)
 
 
+@pytest.mark.parametrize("dims,resident", [((120, 110, 100), True), ((128, 110, 100), False)])
+def test_double_rooms_by_size(gpu, dims, resident):
+    """FP64 rooms beyond about 1.3 M nodes run faster by single steps and take
+    them; on both sides of the line the run equals the z-march kernel."""
+    room = rooms.boxes_room(dims, n_boxes=4, edge=(8, 30), n_materials=5, seed=3)
+    P0 = _values(np.random.default_rng(1), room.n_nodes, "f64")
+    out = []
+    for kernel in ("auto", "zmarch"):
+        with Domain(dims, "f64") as d:
+            d.set_kernel(kernel)
+            d.set_voxels(room.bid, room.mat, centred=False)
+            d.set_materials(room.admittance)
+            d.set_params()
+            d.run(50)
+            d.reset_fields()
+            d.upload_field(L.FIELD_CURRENT, P0)
+            before = L.load().pfdtd_kernel_launches()
+            d.run(15)
+            n = L.load().pfdtd_kernel_launches() - before
+            assert (n <= 2) == (resident and kernel == "auto")
+            out.append((d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
 def test_repeated_run(gpu, O):
     _check(O, (52, 36, 45), "f32", "forward", 33, runs=3)
 
