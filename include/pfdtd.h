@@ -371,12 +371,13 @@ int pfdtd_get_temporal_block(pfdtd_domain* d, int* depth, int* active, char* why
  * A shape that does not exist for the depth makes the next run fail with
  * PFDTD_ERR_ARG. */
 int pfdtd_set_tb_shape(pfdtd_domain* d, int shape);
-/* Autotuner (no counterpart in the reference): times the per-step update and
- * every available (depth <= max_depth, shape) of the blocked update on this
- * domain, `iters` launches each after one warm-up launch, keeps the fastest
+/* Autotuner (no counterpart in the reference): times the unblocked update as
+ * pfdtd_run launches it (per step, or many steps in one launch for a small room
+ * that stays on the SMs) and every available (depth <= max_depth, shape) of the
+ * blocked update on this domain, `iters` launches each after one warm-up launch, keeps the fastest
  * per step on the domain and reports it.  The fields are copied before and
  * restored after the timing launches; node classes are built first.
- * max_depth 0 times the per-step update only. */
+ * max_depth 0 times the unblocked update only. */
 int pfdtd_autotune(pfdtd_domain* d, int max_depth, int iters, int* best_depth, int* best_shape,
                    double* best_ms_per_step);
 

@@ -1187,18 +1187,26 @@ int pfdtd_set_tb_shape(pfdtd_domain* d, int shape) {
 }
 
 // Time one update configuration: `iters` launches after one warm-up launch,
-// returned as milliseconds per step.
+// returned as milliseconds per step.  Without blocking, a room whose runs are
+// resident is timed by such launches.
 static int time_config(pfdtd_domain* d, int iters, double* ms_per_step) {
   cudaStream_t s = d->stream;
   const bool tb = d->tb_depth >= 2 && tb_active(d);
+  bool resident = !tb && resident_usable(d);
   auto launch = [&]() -> int {
     if (tb) return launch_tb(d, nullptr, 0, 0, s);
+    if (resident) return launch_resident(d, 0, d->resident.chunk, nullptr, 0, 0, s);
     int rc = launch_update(d, d->cur_field(), d->past_field(), s);
     d->swap_fields();
     return rc;
   };
   PFDTD_CK(cudaMemsetAsync(d->d_step, 0, sizeof(int64_t), s));
-  if (int rc = launch()) return rc;
+  int rc0 = launch();
+  if (resident && resident_refused(d, rc0)) {
+    resident = false;
+    rc0 = launch();
+  }
+  if (rc0) return rc0;
   cudaEvent_t e0, e1;
   PFDTD_CK(cudaEventCreate(&e0));
   PFDTD_CK(cudaEventCreate(&e1));
@@ -1213,7 +1221,8 @@ static int time_config(pfdtd_domain* d, int iters, double* ms_per_step) {
   cudaEventDestroy(e1);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "autotune timing", __FILE__, __LINE__);
-  *ms_per_step = (double)ms / ((double)iters * (tb ? d->tb_depth : 1));
+  const int64_t steps = tb ? d->tb_depth : resident ? d->resident.chunk : 1;
+  *ms_per_step = (double)ms / ((double)iters * (double)steps);
   return PFDTD_OK;
 }
 

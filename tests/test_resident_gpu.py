@@ -112,6 +112,33 @@ def test_largest_double(gpu, O):
     _check(O, (128, 100, 98), "f64", "forward", 21)
 
 
+@pytest.mark.parametrize("prec", ["f32", "f16"])
+def test_autotune_keeps_resident_runs(gpu, prec):
+    """The autotuner times the resident launches that an automatic run of a
+    small room makes (several times faster than the blocked updates of 64^3) and
+    keeps them; fields and results are as before it."""
+    room, steps = rooms.shoebox((64, 64, 64), seed=1), 60
+    P0 = _values(np.random.default_rng(2), room.n_nodes, prec)
+    with Domain(room.dims, prec) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_receivers([(20, 30, 40)])
+        out = []
+        for tune in (False, True):
+            d.upload_field(L.FIELD_CURRENT, P0)
+            if tune:
+                depth, _, ms = d.autotune(max_depth=4, iters=3)
+                assert depth == 0 and ms > 0
+                assert np.array_equal(d.download_field(L.FIELD_CURRENT), P0)
+            before = L.load().pfdtd_kernel_launches()
+            out.append(d.run(steps)[0])
+            if tune:
+                assert L.load().pfdtd_kernel_launches() - before == 1
+            d.reset_fields()
+    assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("dims,resident", [((120, 110, 100), True), ((128, 110, 100), False)])
 def test_double_rooms_by_size(gpu, dims, resident):
     """FP64 rooms beyond about 1.3 M nodes run faster by single steps and take
