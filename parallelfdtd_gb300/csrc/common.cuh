@@ -457,7 +457,8 @@ int launch_resident(pfdtd_domain* d, int64_t step0, int64_t steps, void* rec_out
                     int64_t inject_end, cudaStream_t s);
 // Implemented in stencil_tb.cu
 int tb_usable(const pfdtd_domain* d, std::string* why);
-int launch_tb(pfdtd_domain* d, void* rec_out, int64_t rec_ld, int64_t inject_end, cudaStream_t s);
+int launch_tb(pfdtd_domain* d, void* rec_out, int64_t rec_ld, int64_t inject_end, cudaStream_t s,
+              int64_t step = -1);
 int check_tb_faces(pfdtd_domain* d);
 bool tb_shape_valid(const pfdtd_domain* d, int shape);
 }  // namespace pfdtd

@@ -117,9 +117,13 @@ int ensure_rec_out(pfdtd_domain* d, int64_t steps) {
 }
 
 // One step on the device: io (record previous, inject this) + update + swap.
+// `step` 0 for the first of a run: the step I/O may start before the operation
+// that it follows has ended, and then does not read the counter, which a memset
+// has just cleared; later ones (-1) read what an earlier step I/O has left, with
+// an update in between.
 int enqueue_step(pfdtd_domain* d, void* rec_out, int64_t rec_ld, int64_t inject_end,
-                 cudaStream_t s) {
-  int rc = launch_io(d, d->cur_field(), rec_out, rec_ld, inject_end, s);
+                 cudaStream_t s, int64_t step = -1) {
+  int rc = launch_io(d, d->cur_field(), rec_out, rec_ld, inject_end, s, 1, step);
   if (rc) return rc;
   rc = launch_update(d, d->cur_field(), d->past_field(), s);
   if (rc) return rc;
@@ -310,11 +314,11 @@ int enqueue_run(pfdtd_domain* d, int64_t steps, void* rec_out, F&& between, bool
   if (rc == PFDTD_OK && !*stopped) {
     int64_t i = 0;
     for (; tb && i + tb <= rem && rc == PFDTD_OK; i += tb) {
-      rc = launch_tb(d, rec_out, steps, steps, s);
+      rc = launch_tb(d, rec_out, steps, steps, s, queued == 0 ? 0 : -1);
       if (rc == PFDTD_OK) queued += tb;
     }
     for (; i < rem && rc == PFDTD_OK; ++i) {
-      rc = enqueue_step(d, rec_out, steps, steps, s);
+      rc = enqueue_step(d, rec_out, steps, steps, s, queued == 0 ? 0 : -1);
       if (rc == PFDTD_OK) ++queued;
     }
   }
@@ -352,9 +356,9 @@ int enqueue_steps(pfdtd_domain* d, int64_t at, int64_t n, void* rec_out, int64_t
     count_launch(d->graph.launches);
   }
   for (; tb && done + tb <= n; done += tb)
-    if (int rc = launch_tb(d, rec_out, rec_ld, inject_end, s)) return rc;
+    if (int rc = launch_tb(d, rec_out, rec_ld, inject_end, s, at + done == 0 ? 0 : -1)) return rc;
   for (; done < n; ++done)
-    if (int rc = enqueue_step(d, rec_out, rec_ld, inject_end, s)) return rc;
+    if (int rc = enqueue_step(d, rec_out, rec_ld, inject_end, s, at + done == 0 ? 0 : -1)) return rc;
   return PFDTD_OK;
 }
 
@@ -926,7 +930,7 @@ int pfdtd_profile_update(pfdtd_domain* d, int iters) {
     // no sources or receivers
     PFDTD_CK(cudaMemsetAsync(d->d_step, 0, sizeof(int64_t), d->stream));
     for (int i = 0; i < iters && rc == PFDTD_OK; ++i)
-      rc = launch_tb(d, nullptr, 0, 0, d->stream);
+      rc = launch_tb(d, nullptr, 0, 0, d->stream, i == 0 ? 0 : -1);
     return rc;
   }
   for (int i = 0; i < iters && rc == PFDTD_OK; ++i) {
@@ -1194,7 +1198,7 @@ static int time_config(pfdtd_domain* d, int iters, double* ms_per_step) {
   const bool tb = d->tb_depth >= 2 && tb_active(d);
   bool resident = !tb && resident_usable(d);
   auto launch = [&]() -> int {
-    if (tb) return launch_tb(d, nullptr, 0, 0, s);
+    if (tb) return launch_tb(d, nullptr, 0, 0, s, 0);  // (no sources: any step)
     if (resident) return launch_resident(d, 0, d->resident.chunk, nullptr, 0, 0, s);
     int rc = launch_update(d, d->cur_field(), d->past_field(), s);
     d->swap_fields();

@@ -94,8 +94,8 @@ int tb_usable(const pfdtd_domain* d, std::string* why) {
 }
 
 int launch_tb(pfdtd_domain* d, void* rec_out, int64_t rec_ld, int64_t inject_end,
-              cudaStream_t s) {
-  int rc = launch_io(d, d->cur_field(), rec_out, rec_ld, inject_end, s, d->tb_depth);
+              cudaStream_t s, int64_t step) {
+  int rc = launch_io(d, d->cur_field(), rec_out, rec_ld, inject_end, s, d->tb_depth, step);
   if (rc) return rc;
   switch (d->precision) {
     case PFDTD_F32: return launch_tb_f32(d, rec_out, rec_ld, inject_end, s);
