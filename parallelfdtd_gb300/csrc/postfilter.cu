@@ -90,6 +90,13 @@ __global__ void __launch_bounds__(kDcThreads) k_dc_block(T* __restrict__ y, int6
     carry_state = Dd{0.0, 0.0};
     carry_x = 0.0;
   }
+  // A state times a power of a; one that is not finite stays as it is, also where
+  // the power has underflowed to 0 (as in the recursion, unless a itself is 0;
+  // the powers are even, so positive).
+  const bool lasting = a != 0.0;
+  auto damped = [&](Dd power, Dd state) {
+    return lasting && not_finite(state.h) ? Dd{state.h, 0.0} : dd_mul(power, state);
+  };
   Dd damp{1.0, 0.0};  // a^(kDcPer lane)
 #pragma unroll
   for (int k = 0; k < 5; ++k)
@@ -117,7 +124,7 @@ __global__ void __launch_bounds__(kDcThreads) k_dc_block(T* __restrict__ y, int6
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       const Dd u = dd_shfl_up(inc, 1 << k);
-      if (lane >= (1 << k)) inc = dd_add(inc, dd_mul(pw.p[k], u));
+      if (lane >= (1 << k)) inc = dd_add(inc, damped(pw.p[k], u));
     }
     Dd in = dd_shfl_up(inc, 1);  // state after the thread before, from the warp's start
     if (lane == 0) in = Dd{0.0, 0.0};
@@ -125,17 +132,17 @@ __global__ void __launch_bounds__(kDcThreads) k_dc_block(T* __restrict__ y, int6
     __syncthreads();
     if (w == 0) {  // the states after each warp, from the tile's start
       Dd s = lane < kWarps ? warp_state[lane] : Dd{0.0, 0.0};
-      if (lane == 0) s = dd_add(s, dd_mul(pw.p[5], carry_state));
+      if (lane == 0) s = dd_add(s, damped(pw.p[5], carry_state));
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const Dd u = dd_shfl_up(s, 1 << k);
-        if (lane >= (1 << k)) s = dd_add(s, dd_mul(pw.p[5 + k], u));
+        if (lane >= (1 << k)) s = dd_add(s, damped(pw.p[5 + k], u));
       }
       if (lane < kWarps) warp_state[lane] = s;
     }
     __syncthreads();
     const Dd before = w == 0 ? carry_state : warp_state[w - 1];
-    in = dd_add(in, dd_mul(damp, before));
+    in = dd_add(in, damped(damp, before));
     __syncthreads();  // every thread has read its samples and the carried values
     // a tile that is not the trace's last is whole
     if (t == kDcThreads - 1) {

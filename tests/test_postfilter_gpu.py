@@ -29,3 +29,28 @@ def test_dc_block_equals_recursion(gpu, n, a, dtype):
     if dtype == np.float32:
         tol = tol + np.finfo(np.float32).eps * np.abs(want)
     assert np.all(np.abs(got.astype(np.float64) - want) <= tol)
+
+
+@pytest.mark.parametrize("a", [0.995, 0.2, 0.0, -0.2, -0.7])
+@pytest.mark.parametrize("at", [5, 16, 511, 9000])
+@pytest.mark.parametrize("what", ["inf", "-inf", "nan", "overflow"])
+def test_dc_block_not_finite(gpu, a, at, what):
+    """A sample that is not finite, or a difference that overflows, leaves the
+    recursion at the same infinities and NaNs for the rest of the trace, however
+    far its powers of a have underflowed; before it the values are finite."""
+    n = 20000
+    x = np.random.default_rng(at).standard_normal(n)
+    if what == "overflow":
+        x[:at], x[at:] = -1.7e308, 1.7e308
+    else:
+        x[at] = float(what)
+    want, xp, yp = np.zeros(n), 0.0, 0.0
+    with np.errstate(all="ignore"):
+        for t in range(n):
+            yp = x[t] - xp + np.float64(a) * yp
+            xp = x[t]
+            want[t] = yp
+    got = pf.fir(x[None], np.array([1.0]), dc_coef=a)[0]
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want))
+    assert np.array_equal(np.isneginf(got), np.isneginf(want))
