@@ -293,6 +293,7 @@ class Domain:
         [n_rec, steps], [(pressure [h, w] float32, node bytes [h, w]), ...]),
         each capture the field after its step.  The copies go to pinned host
         buffers, asynchronously on the domain's stream."""
+        handle = self.handle  # raises on a closed domain, before anything is allocated
         n = len(captures)
         X, Y, Z = self.dims
         shape = lambda o: (Y, X) if o == 0 else ((Z, X) if o == 1 else (Z, Y))
@@ -313,7 +314,7 @@ class Domain:
             pp = (C.c_void_p * max(n, 1))(*[base + 4 * int(o) for o in at[:n]])
             qq = (C.c_void_p * max(n, 1))(*[base + 4 * total + int(o) for o in at[:n]])
             out = np.zeros((max(self.n_rec, 0), steps), dtype=arith_dtype(self.precision))
-            L.call("pfdtd_run_captures", self.handle, int(steps), out.ctypes.data, n,
+            L.call("pfdtd_run_captures", handle, int(steps), out.ctypes.data, n,
                    st.ctypes.data_as(C.POINTER(C.c_int64)),
                    ori.ctypes.data_as(C.POINTER(C.c_int32)),
                    sl.ctypes.data_as(C.POINTER(C.c_int64)), pp, qq)
