@@ -54,3 +54,26 @@ def test_dc_block_not_finite(gpu, a, at, what):
     assert np.array_equal(np.isnan(got), np.isnan(want))
     assert np.array_equal(np.isposinf(got), np.isposinf(want))
     assert np.array_equal(np.isneginf(got), np.isneginf(want))
+
+
+@pytest.mark.parametrize("channels,n", [(3, 699), (3, 700), (3, 701), (3, 719), (3, 720), (3, 721), (3, 1023),
+                                        (3, 1024), (3, 1025), (3, 8207), (3, 8208), (3, 8209), (3, 8704),
+                                        (152, 1000), (153, 1000), (200, 9000), (2000, 300), (5000, 40)])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_dc_block_by_size(gpu, channels, n, dtype):
+    """Few long traces take the block scan, many or short ones a thread each: at
+    sizes on both sides of that line (700 samples of a few channels), of a
+    thread's samples and of a warp's.  Tolerance as above."""
+    a = 0.995
+    x = np.random.default_rng(n).standard_normal((channels, n)).astype(dtype)
+    want = np.zeros((channels, n))
+    xp = yp = np.zeros(channels)
+    for t in range(n):
+        yp = x[:, t].astype(np.float64) - xp + a * yp
+        xp = x[:, t].astype(np.float64)
+        want[:, t] = yp
+    got = pf.fir(x, np.array([1.0]), dc_coef=a)
+    tol = 4 * n * np.finfo(np.float64).eps * np.abs(want).max()
+    if dtype == np.float32:
+        tol = tol + np.finfo(np.float32).eps * np.abs(want)
+    assert np.all(np.abs(got.astype(np.float64) - want) <= tol)
