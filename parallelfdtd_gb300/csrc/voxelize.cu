@@ -31,6 +31,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace pfdtd {
@@ -39,6 +40,7 @@ namespace {
 constexpr int kMaxCrossings = 64;   // triangle crossings per column
 constexpr int kTriTile = 128;       // triangles staged in shared memory per pass
 constexpr int64_t kMostEntries = 32 << 20, kMostCells = 4 << 20;  // of the triangle lists
+constexpr int64_t kFewTris = 64, kFewNodes = 1 << 19;  // that are not binned
 // sampling offsets (fractions of dx) per axis
 constexpr double kEpsX = 1.2345678901e-5, kEpsY = 3.1415926536e-5, kEpsZ = 2.2360679775e-5;
 
@@ -482,6 +484,39 @@ extern "C" int pfdtd_voxelize(const float* vertices, int64_t n_vertices, const u
     int p;
     ~Restore() { if (p >= 0) cudaSetDevice(p); }
   } restore{prev};
+  // Column bins of k_parity's block tiles and node cells of 8^3; both larger (up
+  // to the whole grid, which is the loop over every triangle) where a few large
+  // triangles or a huge grid would make the lists or the cell table too long.  A
+  // few triangles in a small grid are one cell of each kind from the start, whose
+  // list goes up behind the triangles: binning 12 took 75 us of the 399 of a box of
+  // 18^3 nodes.  A call, us, in one cell / binned: 18^3 320 / 399, 66^3 450 / 490, but
+  // 130^3 1300 / 1220, 258^3 4400 / 3750.
+  Bins gc, gn;
+  int64_t ec = n_triangles, en = n_triangles;
+  const bool few = n_triangles <= kFewTris && N <= kFewNodes;
+  if (few) {
+    gc = gn = make_bins(X, Y, Z, X, Y, Z, lo, voxel_edge);
+    std::vector<int> one(2 + (size_t)n_triangles);
+    one[0] = 0;
+    one[1] = (int)n_triangles;
+    for (int t = 0; t < (int)n_triangles; ++t) one[2 + t] = t;
+    const size_t bytes = sizeof(int) * one.size();
+    tris.resize((size_t)n_triangles + (bytes + sizeof(Tri) - 1) / sizeof(Tri));
+    std::memcpy((void*)(tris.data() + n_triangles), one.data(), bytes);
+  } else {
+    for (int64_t m = 1;; m *= 2) {
+      gc = make_bins(X, Y, Z, 32 * m, 4 * m, Z, lo, voxel_edge);
+      ec = bin_entries(gc, tris, kMostEntries);
+      if ((ec <= kMostEntries && bin_cells(gc) <= kMostCells) || bin_cells(gc) == 1) break;
+    }
+    for (int64_t c = 8;; c *= 2) {
+      gn = make_bins(X, Y, Z, c, c, c, lo, voxel_edge);
+      en = bin_entries(gn, tris, kMostEntries);
+      if ((en <= kMostEntries && bin_cells(gn) <= kMostCells) || bin_cells(gn) == 1) break;
+    }
+    if (bin_cells(gc) == 1) ec = n_triangles;
+    if (bin_cells(gn) == 1) en = n_triangles;
+  }
   cudaStream_t s = nullptr;
   PFDTD_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   Tri* d_tris = nullptr;
@@ -498,27 +533,15 @@ extern "C" int pfdtd_voxelize(const float* vertices, int64_t n_vertices, const u
   if (e == cudaSuccess) e = cudaMemsetAsync(d_flags, 0, 2 * sizeof(int), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_smat, 255, N, s);
   int flags[2] = {0, 0};
-  // Column bins of k_parity's block tiles and node cells of 8^3; both larger (up
-  // to the whole grid, which is the loop over every triangle) where a few large
-  // triangles or a huge grid would make the lists or the cell table too long.
-  Bins gc, gn;
-  int64_t ec = 0, en = 0;
-  for (int64_t m = 1;; m *= 2) {
-    gc = make_bins(X, Y, Z, 32 * m, 4 * m, Z, lo, voxel_edge);
-    ec = bin_entries(gc, tris, kMostEntries);
-    if ((ec <= kMostEntries && bin_cells(gc) <= kMostCells) || bin_cells(gc) == 1) break;
-  }
-  for (int64_t c = 8;; c *= 2) {
-    gn = make_bins(X, Y, Z, c, c, c, lo, voxel_edge);
-    en = bin_entries(gn, tris, kMostEntries);
-    if ((en <= kMostEntries && bin_cells(gn) <= kMostCells) || bin_cells(gn) == 1) break;
-  }
-  if (bin_cells(gc) == 1) ec = n_triangles;
-  if (bin_cells(gn) == 1) en = n_triangles;
   int *bc = nullptr, *lc = nullptr, *bn = nullptr, *ln = nullptr;
   if (n_triangles >= INT32_MAX) e = cudaErrorInvalidValue;  // triangle numbers are ints here
-  if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gc, ec, &bc, &lc, s);
-  if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gn, en, &bn, &ln, s);
+  if (few) {
+    bc = bn = (int*)(d_tris + n_triangles);
+    lc = ln = bc + 2;
+  } else {
+    if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gc, ec, &bc, &lc, s);
+    if (e == cudaSuccess) e = build_bins(d_tris, n_triangles, gn, en, &bn, &ln, s);
+  }
   if (e == cudaSuccess) {
     const int64_t tiles = (int64_t)((X + 31) / 32) * ((Y + 3) / 4);
     k_parity<<<(unsigned)tiles, 128, 0, s>>>(d_tris, gc, bc, lc, X, Y, Z, lo[0], lo[1], lo[2],
@@ -549,6 +572,7 @@ extern "C" int pfdtd_voxelize(const float* vertices, int64_t n_vertices, const u
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(bid_out, d_s2, N, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(mat_out, d_m2, N, cudaMemcpyDeviceToHost, s);
+  if (few) bc = lc = bn = ln = nullptr;  // part of d_tris
   for (void* p : {(void*)d_tris, (void*)d_solid, (void*)d_smat, (void*)d_s2, (void*)d_m2,
                   (void*)d_flags, (void*)bc, (void*)lc, (void*)bn, (void*)ln})
     if (p) cudaFreeAsync(p, s);

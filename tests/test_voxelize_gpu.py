@@ -206,3 +206,33 @@ def test_triangle_lists_lose_no_triangle(gpu, nodes, dx, origin):
     ref_bid, ref_mat = _brute_force(v, t, m, dx, dims)
     assert np.array_equal(bid, ref_bid)
     assert np.array_equal(mat, ref_mat)
+
+
+def _tilted_room(nodes, n_obstacles, seed):
+    """A box with octahedra of random corners in it (8 triangles each)."""
+    rng = np.random.default_rng(seed)
+    size = np.array(nodes) - 2.3
+    parts = [box_mesh((0, 0, 0), size, materials=(0, 1, 2, 3, 4, 5))]
+    for k in range(n_obstacles):
+        c, r = size * rng.uniform(0.3, 0.7, 3), size * rng.uniform(0.15, 0.28, (2, 3))
+        p = np.array([c - [r[0, 0], 0, 0], c + [r[1, 0], 0, 0], c - [0, r[0, 1], 0],
+                      c + [0, r[1, 1], 0], c - [0, 0, r[0, 2]], c + [0, 0, r[1, 2]]])
+        p += rng.uniform(-0.05, 0.05, (6, 3)) * size
+        f = [(i, j, l) for i in (0, 1) for j in (2, 3) for l in (4, 5)]
+        parts.append((p.astype(np.float32), np.array(f, np.uint32), np.full(8, 6 + k, np.uint8)))
+    return merge(*parts)
+
+
+@pytest.mark.parametrize("nodes,n_obstacles,more", [
+    ((33, 21, 13), 0, 0), ((33, 21, 13), 2, 0), ((33, 21, 13), 2, 36), ((33, 21, 13), 2, 37),
+    ((33, 5, 9), 9, 0), ((32, 8, 16), 9, 0), ((65, 41, 23), 9, 0), ((6, 5, 4), 9, 0)])
+def test_few_triangles_are_not_binned(gpu, nodes, n_obstacles, more):
+    """Meshes of 12 and 28 triangles, 64 and 65 (with some that no line crosses)
+    and 84, on both sides of where lists per cell start, the last at sizes on
+    either side of the cells, equal a loop over every triangle."""
+    v, t, m = _tilted_room(nodes, n_obstacles, 5)
+    t = np.concatenate([t, np.array([[0, 0, 7]] * more, np.uint32).reshape(-1, 3)])
+    m = np.concatenate([m, np.full(more, 99, np.uint8)])
+    bid, mat, dims, _ = voxelize(v, t, m, 1.0)
+    ref_bid, ref_mat = _brute_force(v, t, m, 1.0, dims)
+    assert np.array_equal(bid, ref_bid) and np.array_equal(mat, ref_mat)
