@@ -236,3 +236,18 @@ def test_few_triangles_are_not_binned(gpu, nodes, n_obstacles, more):
     bid, mat, dims, _ = voxelize(v, t, m, 1.0)
     ref_bid, ref_mat = _brute_force(v, t, m, 1.0, dims)
     assert np.array_equal(bid, ref_bid) and np.array_equal(mat, ref_mat)
+
+
+def test_lists_too_long_take_larger_cells(gpu):
+    """500 triangles across the whole of a 3000 x 3000 x 5 grid would be in more
+    lists than are kept of either kind, so both take larger cells.  No line
+    crosses these triangles (two corners coincide), and the result is that of
+    the mesh without them."""
+    v, t, m = _tilted_room((3000, 3000, 5), 3, 6)
+    far = np.argmax(v.sum(axis=1))
+    near = np.argmin(v.sum(axis=1))
+    more = np.array([[near, near, far]] * 500, np.uint32)
+    want = voxelize(v, t, m, 1.0)
+    got = voxelize(v, np.concatenate([t, more]), np.concatenate([m, np.full(500, 99, np.uint8)]), 1.0)
+    assert want[2] == got[2] == (3000, 3000, 5) and np.count_nonzero(want[0]) > 10 ** 7
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
