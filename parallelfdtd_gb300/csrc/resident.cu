@@ -696,11 +696,12 @@ int launch_nz(pfdtd_domain* d, const Args<S>& a, cudaStream_t s) {
 // 6.4 and 7.0 / 9.0.
 constexpr int kMaxPlanes = 8;
 // Nodes per SM of an FP64 room.  The z-march kernel keeps the FP64 units busier
-// once it fills the SMs.  Forward and centred, us a step, resident / single: 64^3
-// 8.2 / 9.8 and 12.8 / 15.6, 96^3 26.1 / 22.2 and 40.6 / 60.8, 120 x 110 x 100 37.4 / 41.1
-// and 59.7 / 61.1; beyond the line 130 x 100 x 105 42.0 / 40.9 and 65.9 / 64.5, 128^3
-// 57.9 / 49.3 and 93.1 / 78.5.
-constexpr int kMostDoubles = 8700;
+// once it fills the SMs.  Forward and centred, us a step, resident / single: 24^3
+// 3.0 / 3.4 and 4.3 / 4.1, 64^3 8.2 / 9.3 and 12.8 / 14.3, 100 x 90 x 80 22.4 / 26.2 and
+// 37.3 / 44.5, 92 x 90 x 92 20.8 / 22.9 and 33.7 / 38.9; beyond the line 128 x 96 x 64
+// 23.0 / 20.3 and 36.9 / 34.1, 96^3 26.1 / 23.0 and 40.6 / 38.9, 128 x 96 x 100 33.2 / 29.4
+// and 54.2 / 44.6, though 112 x 104 x 100 32.4 / 32.0 and 53.5 / 55.0.
+constexpr int kMostDoubles = 5100;
 
 template <typename S, int SCHEME>
 int launch_scheme(pfdtd_domain* d, const Args<S>& a, cudaStream_t s) {

@@ -326,6 +326,38 @@ __global__ void k_map_classes(const uint8_t* __restrict__ pos, const uint8_t* __
     cls[i] = (C)lut[((unsigned)pos[i] << 8) | mat[i]];
 }
 
+constexpr int kResidentBlocks = 8;  // z-march blocks an SM holds (2048 threads)
+
+// FP64 z-march updates are bound by the SMs' FP64 units, so what counts is that
+// every SM gets the same work.  While all blocks are resident at once, they are
+// dealt out whole: the planes of a chunk, at most `most`, are chosen for the least
+// work on the busiest SM (a chunk's two more planes cost loads only, half a
+// plane).  Us an update of rooms left to single steps, chunks of 8 planes / so:
+// 24^3 9.8 / 3.2, 100 x 90 x 80 29.2 / 26.3, 101 x 103 x 99 36.1 / 32.1, centred 128 x 96 x
+// 100 62.3 / 44.6.
+//
+// For the same reason such a room is launched plainly.  As a programmatic
+// dependent its blocks are placed while those of the kernel before it are still
+// there, two on one SM and none on another: us a step, dependent / plain, 100 x 90 x
+// 80 40.3 / 29.2, centred 96^3 60.6 / 38.8, with DIF walls (whose pass the update
+// follows) 64^3 17.9 / 13.9, 80^3 30.6 / 20.5.  Up to two blocks an SM (without DIF
+// walls, half a block with) there is room beside them, and rooms of more blocks
+// than are resident are dealt out as they go: both gain the gap, 0.7 us.
+int64_t balanced_chunk(int64_t columns, int64_t nz, int64_t most, int sms) {
+  int64_t best_c = most;
+  double best = 1e30;
+  for (int64_t c = most; c >= 1; --c) {
+    const int64_t blocks = columns * ((nz + c - 1) / c), per = (blocks + sms - 1) / sms;
+    if (per > kResidentBlocks) break;
+    const double cost = (double)per * ((double)c + 0.5);
+    if (cost < best - 1e-9) {
+      best = cost;
+      best_c = c;
+    }
+  }
+  return best_c;
+}
+
 template <typename S, typename C, int SCHEME>
 int launch_update_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   using A = typename Store<S>::A;
@@ -338,16 +370,23 @@ int launch_update_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s
   const int64_t target = (int64_t)d->sm_count * 8 * 4;
   int64_t zc = std::max<int64_t>(8, (nz * (int64_t)gx * gy + target - 1) / target);
   zc = std::min<int64_t>(zc, nz);
+  bool dependent = true;
+  if (sizeof(A) == 8) {
+    zc = balanced_chunk((int64_t)gx * gy, nz, zc, d->sm_count);
+    const int64_t blocks = (int64_t)gx * gy * ((nz + zc - 1) / zc);
+    const int64_t even = d->n_dif > 0 ? d->sm_count / 2 : 2 * (int64_t)d->sm_count;
+    dependent = blocks <= even || blocks > kResidentBlocks * (int64_t)d->sm_count;
+  }
   const int gz = (int)((nz + zc - 1) / zc);
   const size_t as = sizeof(A);
   const char* tb = (const char*)d->d_ctab;
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  PFDTD_CK(launch_step_kernel(k_update_zmarch<S, C, SCHEME>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
-                              (const C*)d->d_cls, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y,
-                              d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift,
-                              (unsigned)d->air_class));
+  PFDTD_CK(launch_kernel(dependent, k_update_zmarch<S, C, SCHEME>, dim3(gx, gy, gz), dim3(kBX, kBY),
+                         0, s, (const C*)d->d_cls, (const S*)cur, (S*)past, tab, (int)XE, (int)d->Y,
+                         d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->K, d->kshift,
+                         (unsigned)d->air_class));
   count_launch();
   return PFDTD_OK;
 }

@@ -43,3 +43,40 @@ def test_f64(gpu, O, dims, scheme, kernel, bad):
                        [], steps, scheme=2 if scheme == "centred" else 0, double=True, P0=P0, Pp0=Pp0)
     assert np.array_equal(P, rP, equal_nan=True)
     assert np.array_equal(Pp, rPp, equal_nan=True)
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4), (24, 24, 24), (48, 40, 36), (35, 17, 60), (64, 64, 64),
+                                  (100, 90, 80), (128, 96, 100), (130, 128, 128)])
+@pytest.mark.parametrize("scheme", ["forward", "centred"])
+@pytest.mark.parametrize("dif", [False, True])
+def test_chunks(gpu, O, dims, scheme, dif):
+    """Chunks of 1 to 8 planes, launched plainly or as programmatic dependents,
+    with and without the pass of frequency-dependent walls behind them."""
+    from parallelfdtd_gb300 import materials
+    room = rooms.boxes_room(dims, n_boxes=3, edge=(4, 9), n_materials=4, seed=4) if min(dims) > 16 \
+        else rooms.shoebox(dims, seed=4)
+    n_mat, steps = len(room.admittance), 6
+    rng = np.random.default_rng(dims[0])
+    P0, Pp0 = rng.uniform(-1, 1, room.n_nodes), rng.uniform(-1, 1, room.n_nodes)
+    flags = np.array([m % 2 for m in range(n_mat)], np.int32)
+    filters = materials.dif_table(materials.positive_real_filters(n_mat, 3, seed=2), 3)
+    at, pulse = tuple(n // 2 for n in dims), rng.uniform(-1, 1, (1, steps))
+    with Domain(dims, "f64") as d:
+        d.set_kernel("zmarch")
+        d.set_scheme(scheme)
+        d.set_voxels(room.bid, room.mat, centred=scheme == "centred")
+        d.set_materials(room.admittance)
+        d.set_params()
+        if dif:
+            d.set_dif_filters(flags, filters)
+        d.set_sources([at], [1], pulse)
+        d.set_receivers([at])
+        d.upload_field(L.FIELD_CURRENT, P0)
+        d.upload_field(L.FIELD_PAST, Pp0)
+        got, _, _ = d.run(steps)
+        P, Pp = d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)
+    pos, mat = O.encode_nodes(room.bid, room.mat, scheme == "centred")
+    want, rP, rPp = O.run(pos, mat, dims, room.admittance, default_params(), [room.flat(*at)], [1], pulse,
+                          [room.flat(*at)], steps, scheme=2 if scheme == "centred" else 0, double=True,
+                          P0=P0, Pp0=Pp0, **({"dif": (flags, filters)} if dif else {}))
+    assert np.array_equal(got, want) and np.array_equal(P, rP) and np.array_equal(Pp, rPp)

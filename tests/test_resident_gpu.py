@@ -139,9 +139,9 @@ def test_autotune_keeps_resident_runs(gpu, prec):
     assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("dims,resident", [((120, 110, 100), True), ((128, 110, 100), False)])
+@pytest.mark.parametrize("dims,resident", [((92, 90, 92), True), ((96, 96, 96), False)])
 def test_double_rooms_by_size(gpu, dims, resident):
-    """FP64 rooms beyond about 1.3 M nodes run faster by single steps and take
+    """FP64 rooms beyond about 0.8 M nodes run faster by single steps and take
     them; on both sides of the line the run equals the z-march kernel."""
     room = rooms.boxes_room(dims, n_boxes=4, edge=(8, 30), n_materials=5, seed=3)
     P0 = _values(np.random.default_rng(1), room.n_nodes, "f64")
