@@ -323,8 +323,10 @@ __device__ __forceinline__ void tma_producer(const CUtensorMap* map_cur,
 // BATCHED: the field holds K = 1 << kshift interleaved fields per node (K a
 // multiple of 4): X and XY count elements, a consumer thread's 4 elements are
 // 4 fields of one node, the x neighbours are K elements away and the class
-// ids (one per node) come in a box K times narrower.
-template <typename S, typename C, int SCHEME, typename Lay, bool BATCHED = false>
+// ids (one per node) come in a box K times narrower.  AIR (FP64): a warp in open
+// air leaves out products.
+template <typename S, typename C, int SCHEME, typename Lay, bool BATCHED = false,
+          bool AIR = sizeof(S) == 8>
 __global__ void __launch_bounds__(Lay::THREADS, Lay::MINB)
 k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant__ CUtensorMap map_past,
              const __grid_constant__ CUtensorMap map_cls,
@@ -578,7 +580,7 @@ k_update_tma(const __grid_constant__ CUtensorMap map_cur, const __grid_constant_
           }
         }
         stgv<VEC>(Pp + idx, res);
-      } else if constexpr (sizeof(A) == 8 && SCHEME != 3) {
+      } else if constexpr (AIR && sizeof(A) == 8 && SCHEME != 3) {
         // FP64: an SM issues 1.7 operations a cycle, which bounds this kernel,
         // so a warp whose nodes are all open air (class `air`: a = 1, c = +-1,
         // no boundary axis) leaves out the products by 1 and, centred, the
@@ -852,7 +854,8 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, size_t esize, void* base, 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename S, typename C, int SCHEME, typename Lay, bool BATCHED = false>
+template <typename S, typename C, int SCHEME, typename Lay, bool BATCHED = false,
+          bool AIR = sizeof(S) == 8>
 int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   using A = typename Store<S>::A;
   constexpr int kTX = Lay::TX;
@@ -905,12 +908,12 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   if (!attr_done[d->device].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lock(attr_mu);
     if (!attr_done[d->device].load(std::memory_order_relaxed)) {
-      PFDTD_CK(cudaFuncSetAttribute(k_update_tma<S, C, SCHEME, Lay, BATCHED>,
+      PFDTD_CK(cudaFuncSetAttribute(k_update_tma<S, C, SCHEME, Lay, BATCHED, AIR>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM));
       int occ = 0;
       if (SCHEME == 3)
         PFDTD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ, k_update_tma<S, C, SCHEME, Lay, BATCHED>, Lay::THREADS, Lay::SMEM));
+            &occ, k_update_tma<S, C, SCHEME, Lay, BATCHED, AIR>, Lay::THREADS, Lay::SMEM));
       occupancy[d->device].store(occ, std::memory_order_relaxed);
       attr_done[d->device].store(true, std::memory_order_release);
     }
@@ -924,8 +927,10 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // first stages arrive, about two planes' more (chunks of 16 planes or more
   // left small rooms to a few CTAs: 10 us an update on 48 x 40 x 36, 3.9
   // now).  FP64 is bound by its operations, which the loads do not add to
-  // (100 x 90 x 80, 8 fields: 195 -> 135 us); 16-bit tiles, nearer to that, do
-  // with two planes (448 x 320 x 240 FP16 68.4 -> 63.4 us).
+  // (100 x 90 x 80, 8 fields: 195 -> 135 us), and rooms of a few tiles take chunks
+  // of two planes while every SM has one chunk at most (4 fields of 16^3 13.2 -> 6.2
+  // us); 16-bit tiles, nearer to that, do with two planes more (448 x 320 x 240 FP16
+  // 68.4 -> 63.4 us).
   constexpr int kMinPlanes = 4;
   constexpr double kMorePlanes = sizeof(A) == 8 ? 0.4 : sizeof(S) == 2 ? 2.0 : 4.0;
   const int64_t per_sm =
@@ -936,7 +941,9 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int64_t tiles = (int64_t)gx * gy;
   int64_t best_c = 1;
   double best = 1e30;
-  for (int64_t c = 1; c <= std::max<int64_t>(1, nz / kMinPlanes); ++c) {
+  int64_t most = std::max<int64_t>(1, nz / kMinPlanes);
+  if (sizeof(A) == 8) most = std::max(most, std::min<int64_t>(nz / 2, d->sm_count / tiles));
+  for (int64_t c = 1; c <= most; ++c) {
     const int64_t ctas = tiles * c;
     const int64_t waves = (ctas + resident - 1) / resident;
     const double eff = (double)ctas / (double)(waves * resident);  // wave fill
@@ -955,9 +962,15 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // before drains streams 3 % slower there than its gap costs (512 x 384 x 256:
   // 65.1 us a step, 61.1 plainly; 512 x 384 x 200 centred BF16 74.8, 72.1), while
   // 384 x 320 x 256 takes 43.0 against 45.5.
-  const bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000);
+  // FP64 tiles that are all resident at once, more than one on an SM, are too: set
+  // up beside the step I/O they lie unevenly on the SMs, whose FP64 units bound
+  // them (8 fields of 96^3 forward 162 / 154, centred 287 / 245; see stencil.cu).  (The
+  // form without the shortcut gains the gap, 1 us, all the same.)
+  const int64_t ctas = tiles * gz;
+  const bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000) &&
+                         !(BATCHED && sizeof(A) == 8 && AIR && ctas > d->sm_count && ctas <= resident);
   PFDTD_CK(launch_kernel(
-      dependent, k_update_tma<S, C, SCHEME, Lay, BATCHED>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
+      dependent, k_update_tma<S, C, SCHEME, Lay, BATCHED, AIR>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
       ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur, (S*)past,
       tab, (int)XE, (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, (A)d->params[1], d->d_err,
       d->kshift, SCHEME == 3 ? d->d_iwb_sw : nullptr, -0.0f, d->wait_ns, (unsigned)d->air_class));
@@ -968,6 +981,21 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
 template <typename S, typename Lay8, typename Lay16>
 int launch_tma_batched(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const bool centred = (d->class_scheme == PFDTD_SRL);
+  if constexpr (sizeof(S) == 8) {
+    // FP64: the shortcut of a warp in open air pays from 6 tile columns on.  In
+    // fewer the warps of the two at the walls, where the general form as a function
+    // takes longer than inlined, are too many.  Us a step, with / without: 4 fields of
+    // 128^3 199 / 182, centred 325 / 290 (4 columns), of 160 x 120 x 110 183 / 183 and 324 /
+    // 291 (5), of 200 x 110 x 108 215 / 234 and 297 / 374 (7); 8 fields of 96 x 80 x 60
+    // 79.2 / 81.8 and 115 / 130 (6), of 256 x 40 x 64 104 / 113 and 134 / 180 (16).
+    if (d->X * d->K <= 5 * Lay8::TX) {
+      if (d->cls_bytes == 1)
+        return centred ? launch_tma_t<S, uint8_t, 1, Lay8, true, false>(d, cur, past, s)
+                       : launch_tma_t<S, uint8_t, 0, Lay8, true, false>(d, cur, past, s);
+      return centred ? launch_tma_t<S, uint16_t, 1, Lay16, true, false>(d, cur, past, s)
+                     : launch_tma_t<S, uint16_t, 0, Lay16, true, false>(d, cur, past, s);
+    }
+  }
   if constexpr (std::is_same<S, float>::value) {  // the difference form (FP32 fields)
     if (d->class_form == PFDTD_FORM_DIFFERENCE)
       return d->cls_bytes == 1 ? launch_tma_t<S, uint8_t, 4, Lay8, true>(d, cur, past, s)

@@ -80,3 +80,40 @@ def test_chunks(gpu, O, dims, scheme, dif):
                           [room.flat(*at)], steps, scheme=2 if scheme == "centred" else 0, double=True,
                           P0=P0, Pp0=Pp0, **({"dif": (flags, filters)} if dif else {}))
     assert np.array_equal(got, want) and np.array_equal(P, rP) and np.array_equal(Pp, rPp)
+
+
+@pytest.mark.parametrize("dims,fields", [((8, 8, 8), 4), ((16, 12, 20), 8), ((160, 9, 12), 4), ((164, 9, 12), 4),
+                                         ((80, 9, 14), 8), ((84, 20, 40), 8), ((96, 60, 50), 8), ((300, 8, 8), 4)])
+@pytest.mark.parametrize("scheme", ["forward", "centred"])
+@pytest.mark.parametrize("wide", [False, True])
+def test_batched(gpu, O, dims, fields, scheme, wide):
+    """Several fields, a few tile columns (5 and less) and more, short chunks and
+    long, 8- and 16-bit class ids: every field equals the oracle's run of it
+    alone, also with an infinity in the field."""
+    room = rooms.shoebox(dims, seed=4)
+    rng = np.random.default_rng(dims[0])
+    mat, table = room.mat, room.admittance
+    if wide:  # more than 256 classes
+        table = rooms.admittance_table(100, 0.05, 0.9, 9)
+        mat = np.where(room.bid > 0, rng.integers(0, 100, room.n_nodes), 0).astype(np.uint8)
+    P0, Pp0 = rng.uniform(-1, 1, (2, room.n_nodes, fields))
+    P0[room.flat(*(n // 2 for n in dims)), 1] = np.inf
+    steps = 3  # the value reaches no wall
+    with Domain(dims, "f64", fields=fields) as d:
+        d.set_scheme(scheme)
+        d.set_voxels(room.bid, mat, centred=scheme == "centred")
+        d.set_materials(table)
+        d.set_params()
+        d.upload_field(L.FIELD_CURRENT, P0.reshape(-1))
+        d.upload_field(L.FIELD_PAST, Pp0.reshape(-1))
+        d.run(steps)
+        P = d.download_field(L.FIELD_CURRENT).reshape(-1, fields)
+        Pp = d.download_field(L.FIELD_PAST).reshape(-1, fields)
+        assert d.kernel() == "tma"
+    pos, m = O.encode_nodes(room.bid, mat, scheme == "centred")
+    for f in (0, 1, fields - 1):
+        _, rP, rPp = O.run(pos, m, dims, table, default_params(), [], [], np.zeros((0, steps)), [], steps,
+                           scheme=2 if scheme == "centred" else 0, double=True,
+                           P0=np.ascontiguousarray(P0[:, f]), Pp0=np.ascontiguousarray(Pp0[:, f]))
+        assert np.array_equal(P[:, f], rP, equal_nan=True), f
+        assert np.array_equal(Pp[:, f], rPp, equal_nan=True), f
