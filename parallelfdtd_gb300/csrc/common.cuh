@@ -447,6 +447,8 @@ int launch_iwb_tma(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s)
 bool uses_tma(const pfdtd_domain* d);
 // Implemented in stencil_flat.cu
 bool flat_usable(const pfdtd_domain* d);
+bool flat_pays(const pfdtd_domain* d);
+bool full_runs(const pfdtd_domain* d);
 bool iwb_flat(const pfdtd_domain* d);
 int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s);
 bool prefers_flat(const pfdtd_domain* d);  // stencil_tma.cu

@@ -1143,7 +1143,7 @@ int pfdtd_set_tile(pfdtd_domain* d, int tile) {
 int pfdtd_get_kernel(pfdtd_domain* d, int* variant) {
   if (int rc = check_domain(d)) return rc;
   if (!variant) return fail(PFDTD_ERR_ARG, "null output");
-  const bool flat = d->class_scheme == PFDTD_IWB ? iwb_flat(d) : flat_usable(d);
+  const bool flat = d->class_scheme == PFDTD_IWB ? iwb_flat(d) : flat_pays(d);
   *variant = uses_tma(d) || flat ? PFDTD_KERNEL_TMA : PFDTD_KERNEL_ZMARCH;
   if (d->tb_depth >= 2 && tb_active(d)) *variant = PFDTD_KERNEL_TB;
   return PFDTD_OK;

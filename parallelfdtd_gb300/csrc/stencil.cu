@@ -460,7 +460,7 @@ int launch_update(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) 
     if (d->class_scheme == PFDTD_IWB) return launch_iwb_tma(d, cur, past, s);
     return prefers_flat(d) ? launch_update_flat(d, cur, past, s) : launch_update_tma(d, cur, past, s);
   }
-  if (d->class_scheme != PFDTD_IWB && flat_usable(d)) return launch_update_flat(d, cur, past, s);
+  if (d->class_scheme != PFDTD_IWB && flat_pays(d)) return launch_update_flat(d, cur, past, s);
   switch (d->precision) {
     case PFDTD_F32: return launch_update_s<float>(d, cur, past, s);
     case PFDTD_F64: return launch_update_s<double>(d, cur, past, s);

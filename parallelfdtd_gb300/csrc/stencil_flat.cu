@@ -514,19 +514,49 @@ bool flat_usable(const pfdtd_domain* d) {
   return d->X * d->K <= 4096 && d->XY * d->K < ((int64_t)1 << 31) && flat_stages(d) >= 4;
 }
 
+// Whether a plane's last run is full enough: with 13 x 13 nodes of a run of 2048
+// (1.5 M nodes in 9000 planes) an update took 32.7 us, 12.2 by the z-march kernel.
+bool full_runs(const pfdtd_domain* d) {
+  const int64_t n = d->XY * d->K;
+  return 4 * n >= 3 * ((n + kRange - 1) / kRange) * kRange;
+}
+
+// Whether a 7-point room whose rows are not aligned takes the flat runs, or the
+// z-march kernel: a CTA's stage ring only pays once there are enough runs to share.
+// Us a step by single steps, FP32, z-march / runs: forward 50 x 41 x 36 4.9 / 6.3, 81 x
+// 80 x 79 5.3 / 6.2, 90 x 91 x 89 (0.73 M) 5.7 / 6.3, two fields of 701 x 30 x 20 (0.84 M)
+// 6.6 / 6.6, 97^3 (0.91 M) 8.0 / 6.2, 203 x 155 x 119 12.1 / 10.6; centred 5.2 / 8.1, 5.6 /
+// 8.0, 5.8 / 8.1, 7.2 / 7.3, 9.1 / 8.0, 14.0 / 13.0; 16-bit fields alike.  Centred
+// updates take longer a plane, and where some SMs have two CTAs and most one, or a
+// chunk is all of a few planes, the runs lose: two fields of 96^3 (171 CTAs) 9.5 / 9.9,
+// 131 x 127 x 125 (225) 9.8 / 10.5, two of 400 x 300 x 8 8.0 / 9.1; with 250 CTAs and more
+// they win (161 x 120 x 110, 270: 9.8 / 8.8).
+bool flat_pays(const pfdtd_domain* d) {
+  if (!flat_usable(d)) return false;
+  if (d->kernel_variant == PFDTD_KERNEL_TMA) return true;
+  if (d->N * d->K < 850000 || !full_runs(d)) return false;
+  if (d->class_scheme != PFDTD_SRL) return true;
+  const int64_t nz = d->Z - 2, gx = (d->XY * d->K + kRange - 1) / kRange, zc = flat_chunk(d, gx);
+  const int64_t ctas = gx * ((nz + zc - 1) / zc);
+  return nz >= 8 && (ctas <= d->sm_count || 10 * ctas >= 16 * (int64_t)d->sm_count);
+}
+
 // Whether the next IWB update is by flat runs with the closure pass.
-// Measured with DIF walls, us a step.  Rows that are not aligned, z-march / runs,
-// FP32: 203 x 155 x 119 33.6 / 19.6, 401 x 301 x 201 227 / 70.3, 131 x 127 x 125 24.0 /
-// 16.2; from about a million nodes (97 x 81 x 65 13.3 / 15.2), below which the
-// closure pass costs more than the update saves.  Aligned rows, tiles / runs, FP32:
+// Measured, us a step, FP32.  Rows that are not aligned, z-march / runs, with DIF
+// walls: 97 x 81 x 65 11.9 / 13.9, 90 x 91 x 89 11.7 / 14.2, 101 x 103 x 99 (1.03 M) 15.3 /
+// 14.6, 203 x 155 x 119 29.8 / 18.0; without, where the closure pass is all loss, 101 x
+// 103 x 99 12.2 / 14.4, 401 x 300 x 12 (1.44 M) 10.9 / 13.5, 45 x 45 x 1000 (2.03 M) 22.3 /
+// 15.5, 131 x 127 x 125 18.1 / 14.8.  Aligned rooms, tiles / runs, FP32 with DIF walls:
 // 160^3 28.5 / 22.8, 384 x 320 x 256 103.9 / 91.6, 512 x 384 x 256 144.9 / 136.6,
 // 256 x 192 x 128 29.7 / 29.3, 128^3 no difference (without walls 17.0 / 18.2); in
 // FP16 512 x 384 x 256 without walls 150.6 / 157.2.
 bool iwb_flat(const pfdtd_domain* d) {
   if (d->class_scheme != PFDTD_IWB || !flat_usable(d)) return false;
-  if (!uses_tma(d)) return d->kernel_variant == PFDTD_KERNEL_TMA || d->N >= 1000000;
+  if (!uses_tma(d))
+    return d->kernel_variant == PFDTD_KERNEL_TMA ||
+           (d->N >= (d->n_dif > 0 ? 1000000 : 1600000) && full_runs(d));
   return d->kernel_variant == PFDTD_KERNEL_AUTO && d->tma_tile < 0 && d->precision == PFDTD_F32 &&
-         d->N >= 3000000;
+         d->N >= 3000000 && full_runs(d);
 }
 
 int launch_update_flat(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {

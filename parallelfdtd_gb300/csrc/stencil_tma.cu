@@ -1239,7 +1239,7 @@ bool iwb_closure_fuses_dif(const pfdtd_domain* d) {
 // 15.7 / 15.4; 176^3 15.6 / 15.4, centred 18.2 / 20.4; 320 x 200 x 160 22.5 / 24.0).
 bool prefers_flat(const pfdtd_domain* d) {
   if (d->kernel_variant != PFDTD_KERNEL_AUTO || d->tma_tile >= 0 || d->K != 1) return false;
-  if (d->class_scheme == PFDTD_IWB || d->N < 3000000 || !flat_usable(d)) return false;
+  if (d->class_scheme == PFDTD_IWB || d->N < 3000000 || !flat_usable(d) || !full_runs(d)) return false;
   if (d->precision != PFDTD_F32) return auto_tile16(d) == 0 && d->N < 5000000;
   return auto_tile(d) != 6 || (d->class_scheme != PFDTD_SRL && d->N >= 8000000);
 }

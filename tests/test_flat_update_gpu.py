@@ -179,3 +179,39 @@ def test_iwb(gpu, O, prec, dims, wide):
     want, rP, rPp = O.run(pos, m, dims, table, params, src, [1, 1], pulses, rec, steps, scheme=3,
                           storage=None if prec == "f32" else prec, dif=(flags, filters), P0=P0, Pp0=Pp0)
     assert np.array_equal(got, want) and np.array_equal(P, rP) and np.array_equal(Pp, rPp)
+
+
+@pytest.mark.parametrize("dims,scheme,fields,dif,flat", [
+    ((90, 91, 89), "forward", 1, False, False), ((97, 97, 97), "forward", 1, False, True),
+    ((97, 97, 97), "centred", 1, False, True), ((13, 13, 5100), "centred", 1, False, False),
+    ((96, 96, 96), "centred", 2, False, False), ((161, 120, 110), "centred", 1, False, True),
+    ((80, 80, 66), "forward", 2, False, False), ((80, 80, 68), "forward", 2, False, True),
+    ((90, 91, 89), "iwb", 1, True, False), ((101, 103, 99), "iwb", 1, True, True),
+    ((101, 103, 99), "iwb", 1, False, False), ((131, 127, 101), "iwb", 1, False, True),
+    ((13, 13, 9600), "iwb", 1, False, False)])
+def test_rooms_by_size(gpu, dims, scheme, fields, dif, flat):
+    """Rooms whose rows are not aligned (or with two fields) take the runs from
+    where they pay, the z-march kernel below and where a plane fills too little of
+    a run, and both give the z-march kernel's fields."""
+    from parallelfdtd_gb300 import materials
+    room = rooms.boxes_room(dims, n_boxes=3, edge=(8, 30), n_materials=5, seed=3) if min(dims) > 40 \
+        else rooms.shoebox(dims, seed=3)
+    P0 = _values(np.random.default_rng(1), room.n_nodes * fields, "f32")
+    out, n_mat = [], len(room.admittance)
+    for kernel in ("auto", "zmarch"):
+        with Domain(dims, fields=fields) as d:
+            d.set_kernel(kernel)
+            d.set_scheme(scheme)
+            d.set_voxels(room.bid, room.mat, centred=scheme != "forward")
+            d.set_materials(room.admittance)
+            d.set_params(default_params(scheme="iwb" if scheme == "iwb" else "forward"))
+            if dif:
+                d.set_dif_filters(np.array([m % 2 for m in range(n_mat)], np.int32),
+                                  materials.dif_table(materials.positive_real_filters(n_mat, 3, seed=2), 3))
+            d.upload_field(L.FIELD_CURRENT, P0)
+            L.call("pfdtd_run_async", d.handle, 5)  # by single steps
+            d.synchronize()
+            assert d.kernel() == ("tma" if flat and kernel == "auto" else "zmarch")
+            out.append((d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
