@@ -408,10 +408,16 @@ int launch_iwb_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  PFDTD_CK(launch_step_kernel(k_update_iwb<S, C>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
-                              (const C*)d->d_cls, d->d_iwb_mask, (const S*)cur, (S*)past, tab, (int)XE,
-                              (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, d->K, d->kshift,
-                              (A)d->params[1]));
+  // (of up to two blocks an SM, all resident at once, some would lie on one SM as
+  // programmatic dependents: 81 x 80 x 79 8.8 us a step, plainly 7.5.  A DIF pass in
+  // between leaves more time: 10.3 and 10.6.)
+  const int64_t blocks = (int64_t)gx * gy * gz;
+  const bool dependent =
+      d->n_dif > 0 || 2 * blocks <= 3 * (int64_t)d->sm_count || blocks > 2 * (int64_t)d->sm_count;
+  PFDTD_CK(launch_kernel(dependent, k_update_iwb<S, C>, dim3(gx, gy, gz), dim3(kBX, kBY), 0, s,
+                         (const C*)d->d_cls, d->d_iwb_mask, (const S*)cur, (S*)past, tab, (int)XE,
+                         (int)d->Y, d->XY * d->K, (int)(d->Z - 1), (int)zc, d->K, d->kshift,
+                         (A)d->params[1]));
   count_launch();
   return PFDTD_OK;
 }
