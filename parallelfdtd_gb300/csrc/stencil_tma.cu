@@ -962,13 +962,25 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // before drains streams 3 % slower there than its gap costs (512 x 384 x 256:
   // 65.1 us a step, 61.1 plainly; 512 x 384 x 200 centred BF16 74.8, 72.1), while
   // 384 x 320 x 256 takes 43.0 against 45.5.
-  // FP64 tiles that are all resident at once, more than one on an SM, are too: set
-  // up beside the step I/O they lie unevenly on the SMs, whose FP64 units bound
-  // them (8 fields of 96^3 forward 162 / 154, centred 287 / 245; see stencil.cu).  (The
-  // form without the shortcut gains the gap, 1 us, all the same.)
   const int64_t ctas = tiles * gz;
-  const bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000) &&
-                         !(BATCHED && sizeof(A) == 8 && AIR && ctas > d->sm_count && ctas <= resident);
+  bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000);
+  // So are tiles of which all are resident at once, but not as many as fit: set up
+  // beside the kernel before they lie unevenly, two on one SM and none on another.
+  // Us a step, dependent / plain: FP32, 4 fields of 256 x 128 x 96 (256 CTAs of 47 planes
+  // for 304 places) 28.3 / 23.7, of 128^3 (32 planes) 17.7 / 16.5, 8 of 256 x 64 x 64 17.2 /
+  // 16.0; also where they do fit, if long: 8 of 64 x 64 x 400 (288, 45) 28.3 / 24.1, FP16 8
+  // of 192 x 192 x 128 (288, 63) 47.7 / 45.8.  Shorter ones gain the gap: 4 of 64 x 64 x 400
+  // (304, 21) 11.8 / 12.7, 8 of 64^3 (288, 7) 6.5 / 7.1.  IWB tiles, with the closure pass
+  // in between: 400 x 300 x 8 (152) 13.1 / 11.9, 96^3 (276) 13.0 / 12.6; single 7-point
+  // fields gain the gap at all sizes.
+  if (SCHEME == 3 && ctas >= d->sm_count && ctas <= 2 * (int64_t)d->sm_count) dependent = false;
+  if (BATCHED && sizeof(A) == 4 && 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident &&
+      (zc >= 45 || (zc >= 16 && 10 * ctas <= 9 * resident)))
+    dependent = false;
+  // FP64 units bound FP64 tiles, so any unevenness costs (8 fields of 96^3 forward 162 /
+  // 154, centred 287 / 245; see stencil.cu); the form without the shortcut gains the
+  // gap, 1 us, all the same.
+  if (BATCHED && sizeof(A) == 8 && AIR && ctas > d->sm_count && ctas <= resident) dependent = false;
   PFDTD_CK(launch_kernel(
       dependent, k_update_tma<S, C, SCHEME, Lay, BATCHED, AIR>, dim3(gx, gy, gz), dim3(Lay::THREADS), Lay::SMEM, s,
       ts.halo[cur_i], ts.tile[past_i], ts.cls, Lay::MASK ? ts.mask : ts.cls, (const S*)cur, (S*)past,
