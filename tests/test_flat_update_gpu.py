@@ -215,3 +215,35 @@ def test_rooms_by_size(gpu, dims, scheme, fields, dif, flat):
             out.append((d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
 
+
+@pytest.mark.parametrize("prec", ["f16", "bf16"])
+@pytest.mark.parametrize("scheme", ["forward", "centred"])
+@pytest.mark.parametrize("dims,fields", [((37, 29, 18), 4), ((33, 31, 9), 2), ((9, 9, 30), 4)])
+def test_fields_in_16_bits(gpu, O, prec, scheme, dims, fields):
+    _check(O, dims, prec, scheme, fields=fields)
+
+
+@pytest.mark.parametrize("dims", [(160, 128, 120), (256, 96, 101)])
+def test_difference_form_of_tiles(gpu, O, dims):
+    """The difference form in the tiled update, which aligned single-field rooms
+    between the resident and the large ones take."""
+    room = rooms.boxes_room(dims, n_boxes=3, edge=(8, 30), n_materials=5, seed=3)
+    rng = np.random.default_rng(2)
+    P0, Pp0 = _values(rng, room.n_nodes, "f32"), _values(rng, room.n_nodes, "f32")
+    steps, at, pulse = 6, (40, 50, 60), rng.uniform(-1, 1, (1, 6))
+    with Domain(dims) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_update_form("difference")
+        d.set_sources([at], [1], pulse)
+        d.set_receivers([at])
+        d.upload_field(L.FIELD_CURRENT, P0)
+        d.upload_field(L.FIELD_PAST, Pp0)
+        got, _, st = d.run(steps)
+        assert st == 0 and d.kernel() == "tma"
+        P, Pp = d.download_field(L.FIELD_CURRENT), d.download_field(L.FIELD_PAST)
+    pos, mat = O.encode_nodes(room.bid, room.mat, False)
+    want, rP, rPp = O.run(pos, mat, dims, room.admittance, default_params(), [room.flat(*at)], [1], pulse,
+                          [room.flat(*at)], steps, P0=P0, Pp0=Pp0, form="difference")
+    assert np.array_equal(got, want) and np.array_equal(P, rP) and np.array_equal(Pp, rPp)
