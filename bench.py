@@ -499,6 +499,9 @@ def main():
     in_kernel_closure = os.environ.get("PFDTD_TMA_TILE", "-1").strip() in ("0", "1", "2", "3", "4", "5")
     if a.scheme == "iwb" and d.kernel() == "tma" and not in_kernel_closure:
         kernel_name += " + k_iwb_closure"  # the update of a step: both kernels, timed together
+    if T == 1 and launches < a.steps * S:
+        # the run stays on the SMs; what is timed alone is the update of a single step
+        kernel_name += " (single steps; the run itself is k_resident)"
 
     # ---- end to end through the C ABI with host buffers ------------------------
     out_host = np.zeros((n_rec, S), dtype=np.float64 if prec == "f64" else np.float32)

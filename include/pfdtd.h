@@ -191,7 +191,8 @@ int pfdtd_set_scheme(pfdtd_domain* d, int scheme);
  *   16-bit storage the storage rounding dominates and the form gains
  *   nothing); no frequency-dependent boundaries and no temporal blocking
  *   (PFDTD_ERR_UNSUPPORTED at the next run).  */
-/* Bound, in nanoseconds, of each pipeline wait inside the TMA update kernels
+/* Bound, in nanoseconds, of each pipeline wait inside the update kernels and of
+ * each wait for a neighbour's values in a run that stays on the SMs
  * (no counterpart in the reference; default 2 s, 0 restores it).  A wait that
  * runs out raises the domain's error flag; the kernel stops issuing loads,
  * waits for the loads already in flight (always with the 2 s bound) and
@@ -210,7 +211,15 @@ int pfdtd_set_update_form(pfdtd_domain* d, int form);
  * out: host buffer [n_rec * steps] in the arithmetic type, row per receiver.
  * The interrupt callback is polled and the progress callback called every
  * 100 steps.  seconds_per_step (optional) receives wall time / steps.
- * Returns PFDTD_INTERRUPTED if stopped early (rows hold the steps done). */
+ * Returns PFDTD_INTERRUPTED if stopped early (rows hold the steps done).
+ * A small room stays on the SMs for many steps (one launch of about a
+ * millisecond's steps, or 50 with a callback): one field, forward or centred,
+ * kernel, tile and blocking left automatic, outside x and y faces, no
+ * frequency-dependent walls, at most 32 sources and 128 receivers, none on planes
+ * 0 and Z-1, up to about 2.4 M nodes (FP64 0.8 M).  Results are the same while the
+ * fields are finite (a zero on an outside face may differ in sign; a value that is
+ * not finite on such a face reaches the next row's or plane's first node, its
+ * flat-index neighbour, by single steps only). */
 int pfdtd_run(pfdtd_domain* d, int64_t steps, void* out, pfdtd_interrupt_fn interrupt_cb,
               pfdtd_progress_fn progress_cb, double* seconds_per_step);
 
@@ -292,8 +301,9 @@ int pfdtd_run_async(pfdtd_domain* d, int64_t steps);
  * copy each slice synchronously): capture i is the slice cap_slice[i] of
  * orientation cap_orientation[i] (0 xy, 1 xz, 2 yz, as pfdtd_capture_slice)
  * of the field after cap_step[i] steps (0 <= cap_step[i] <= steps).  The
- * run is split at the capture steps, whole chunks still replay their CUDA
- * graphs, and each capture is a gather kernel and an asynchronous copy into
+ * run is split at the capture steps; the pieces are launched as pfdtd_run does (a
+ * small room stays on the SMs where they are long enough on average, otherwise
+ * whole chunks replay their CUDA graphs), and each capture is a gather kernel and an asynchronous copy into
  * p_out[i] (floats) and pos_out[i] (node bytes) on the domain's stream
  * (either array, or one of its entries, may be null).  Pinned host buffers
  * (pfdtd_host_alloc) keep the copies asynchronous.  Receivers as pfdtd_run. */
@@ -306,14 +316,16 @@ int pfdtd_host_free(void* ptr);
 int pfdtd_query(pfdtd_domain* d, int* done);
 int pfdtd_fetch_receivers(pfdtd_domain* d, void* out);
 
-/* Update kernel variant: 0 automatic (a bulk-copy pipelined kernel: TMA tiles
- * when the field rows are 16-byte aligned, X * fields * element size a multiple
- * of 16, class-id rows that are not being read from a padded copy; runs of flat
- * indices for other FP32 and 16-bit rooms with the 7-point schemes, and for
- * large ones; a single FP64 field takes the z-march kernel), 1 the
- * register z-marching kernel, 2 the pipelined kernels.  pfdtd_get_kernel reports the
- * variant the next launch will use (1 or 2, or 3 when the temporally blocked
- * kernel of pfdtd_set_temporal_block will run). */
+/* Update kernel variant: 0 automatic, 1 the register z-marching kernel, 2 the
+ * pipelined bulk-copy kernels, TMA tiles or runs of flat indices.  Automatic takes,
+ * by size, alignment and precision: tiles where the field rows are 16-byte aligned
+ * (X * fields * element size a multiple of 16; class-id rows that are not are read
+ * from a padded copy); runs for large rooms, aligned or not; the z-march kernel for
+ * smaller rooms that are not aligned and for a single FP64 field.
+ * pfdtd_get_kernel reports the variant of the next step launched by itself (1 or 2),
+ * or 3 when the temporally blocked kernel of pfdtd_set_temporal_block will run.
+ * Automatic runs of small rooms need no such launch (see pfdtd_run);
+ * pfdtd_kernel_launches tells them apart. */
 #define PFDTD_KERNEL_AUTO 0
 #define PFDTD_KERNEL_ZMARCH 1
 #define PFDTD_KERNEL_TMA 2

@@ -30,9 +30,10 @@
 //
 // Arithmetic, order and rounding are those of k_update_tma (packed pairs with
 // uncontractible products), so every result is the same.  As in the temporally
-// blocked kernels the x and y faces must lie outside the room (then the
-// flat-index wrap of the reference cannot matter; a zero there may differ in
-// sign).  Every poll is bounded (the domain's wait limit): on expiry the kernel
+// blocked kernels the x and y faces must lie outside the room: then the
+// flat-index wrap of the reference cannot matter while the fields are finite (a
+// zero there may differ in sign; a NaN or an infinity that has reached a face goes
+// on to the wrapped neighbour only by single steps).  Every poll is bounded (the domain's wait limit): on expiry the kernel
 // raises the error flag and returns, and the host reports it.
 #include "common.cuh"
 
