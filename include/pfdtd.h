@@ -215,11 +215,12 @@ int pfdtd_set_update_form(pfdtd_domain* d, int form);
  * A small room stays on the SMs for many steps (one launch of about a
  * millisecond's steps, or 50 with a callback): one field, forward or centred,
  * kernel, tile and blocking left automatic, outside x and y faces, no
- * frequency-dependent walls, at most 32 sources and 128 receivers, none on planes
- * 0 and Z-1, up to about 2.4 M nodes (FP64 0.8 M).  Results are the same while the
- * fields are finite (a zero on an outside face may differ in sign; a value that is
- * not finite on such a face reaches the next row's or plane's first node, its
- * flat-index neighbour, by single steps only). */
+ * frequency-dependent walls, finite samples, passive materials, lambda within its
+ * limit, at most 32 sources and 128 receivers, none on planes 0 and Z-1, up to
+ * about 2.4 M nodes (FP64 0.8 M).  Results are the same, except that a zero on an
+ * outside face may differ in sign, and that a value in the uploaded fields which is
+ * not finite does not pass from a face to its flat-index neighbour in the next row
+ * or plane, as it does by single steps. */
 int pfdtd_run(pfdtd_domain* d, int64_t steps, void* out, pfdtd_interrupt_fn interrupt_cb,
               pfdtd_progress_fn progress_cb, double* seconds_per_step);
 

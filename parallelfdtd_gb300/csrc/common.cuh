@@ -316,6 +316,7 @@ struct pfdtd_domain {
   int class_form = 0;        // update form the class table was built for
   int n_classes = 0;
   int air_class = -1;        // a class of open air (loss-free, no missing neighbour)
+  bool passive = false;      // no class gains energy, lambda within the 7-point limit
   int cls_bytes = 1;
   void* d_cls = nullptr;     // per node class id (uint8 or uint16)
   // The class ids with every row padded to a multiple of 16 bytes, for the
@@ -359,6 +360,7 @@ struct pfdtd_domain {
   std::vector<int64_t> src_idx_h;
   std::vector<int32_t> src_type_h;
   std::vector<uint8_t> src_samples_h;
+  bool src_finite = true;          // every sample, as the fields store it
   int n_rec = 0;
   int64_t* d_rec_idx = nullptr;
   std::vector<int64_t> rec_idx_h;

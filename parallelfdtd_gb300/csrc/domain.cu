@@ -11,6 +11,8 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cfloat>
+#include <cmath>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -663,6 +665,12 @@ int pfdtd_set_sources_batched(pfdtd_domain* d, int n, const int64_t* xyz, const 
   }
   const size_t sbytes = (size_t)n * (size_t)n_samples * d->arith_size();
   d->src_samples_h.assign((const uint8_t*)samples, (const uint8_t*)samples + sbytes);
+  d->src_finite = true;
+  const double most = d->precision == PFDTD_F16 ? 65504.0 : DBL_MAX;  // of the stored field
+  for (size_t i = 0; i < (size_t)n * (size_t)n_samples && d->src_finite; ++i) {
+    const double v = d->precision == PFDTD_F64 ? ((const double*)samples)[i] : ((const float*)samples)[i];
+    d->src_finite = std::fabs(v) <= most;
+  }
   const size_t n1 = std::max(n, 1);
   PFDTD_CK(d->alloc((void**)&d->d_src_idx, n1 * sizeof(int64_t)));
   PFDTD_CK(d->alloc((void**)&d->d_src_mode, n1 * sizeof(int32_t)));

@@ -32,8 +32,10 @@
 // uncontractible products), so every result is the same.  As in the temporally
 // blocked kernels the x and y faces must lie outside the room: then the
 // flat-index wrap of the reference cannot matter while the fields are finite (a
-// zero there may differ in sign; a NaN or an infinity that has reached a face goes
-// on to the wrapped neighbour only by single steps).  Every poll is bounded (the domain's wait limit): on expiry the kernel
+// zero there may differ in sign).  A NaN or an infinity on a face goes on to the
+// wrapped neighbour, so a room that can be foreseen to meet one (samples, materials,
+// lambda) takes single steps; one that a caller has written into a field does not
+// reach that neighbour here.  Every poll is bounded (the domain's wait limit): on expiry the kernel
 // raises the error flag and returns, and the host reports it.
 #include "common.cuh"
 
@@ -778,6 +780,7 @@ bool resident_usable(pfdtd_domain* d) {
   if (d->K != 1 || d->Z < 3 || !d->tb_faces_ok || d->n_dif > 0) return false;
   if (d->class_scheme != PFDTD_SRL_FORWARD && d->class_scheme != PFDTD_SRL) return false;
   if (d->cls_bytes != 1 || d->n_classes > 255) return false;  // one id for nodes past the grid
+  if (!d->passive || !d->src_finite) return false;  // values that are not finite: see above
   if (d->n_src > kMaxSources || d->n_rec > kMaxReceivers) return false;
   if (d->N > (int64_t)d->sm_count * (d->precision == PFDTD_F64 ? kMostDoubles : 40000)) return false;
   for (int64_t e : d->src_idx_h)

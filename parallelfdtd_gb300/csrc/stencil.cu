@@ -520,6 +520,18 @@ static int find_air(int scheme, const std::vector<uint16_t>& keys, const std::ve
   return -1;
 }
 
+// Whether no class of the 7-point schemes gains energy or is not finite: a =
+// s/(1 + beta) and c = 1 - beta (centred beta - 1) of a beta from 0 on.
+template <typename A>
+static bool passive_classes(int scheme, size_t n, const std::vector<uint8_t>& tab) {
+  const A* a = (const A*)tab.data();
+  const A* c = a + 2 * n;
+  const A sign = scheme == PFDTD_SRL ? (A)-1 : (A)1;
+  for (size_t i = 0; i < n; ++i)
+    if (!(a[i] >= (A)0 && a[i] <= (A)1 && sign * c[i] <= (A)1)) return false;
+  return true;
+}
+
 // Whether the IWB classes outside the room and without closed neighbours (codes
 // 0 and 1) have the coefficients these codes stand for; a material that is not
 // finite makes others.
@@ -651,6 +663,10 @@ int build_classes(pfdtd_domain* d) {
                                                 : find_air<float>(scheme, keys, tab);
   d->iwb_open = scheme == PFDTD_IWB && d->precision != PFDTD_F64 &&
                 iwb_open_classes(keys, tab, &d->iwb_open_b);
+  // (1e-5 for a lambda rounded to float)
+  d->passive = d->params[1] <= (1.0 / 3.0) * (1.0 + 1e-5) &&
+               (d->precision == PFDTD_F64 ? passive_classes<double>(scheme, keys.size(), tab)
+                                          : passive_classes<float>(scheme, keys.size(), tab));
   d->class_scheme = scheme;
   d->class_form = form;
   rc = build_dif(d, keys, tab);

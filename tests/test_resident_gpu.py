@@ -332,3 +332,60 @@ def test_refused_cooperative_launch(gpu, tmp_path, code):
     assert got["launches"] > 3 * 2 * 70  # update and step I/O of every step
     for i, v in enumerate(_refusal_run()):
         assert np.array_equal(got["arr_%d" % i], v), i
+
+
+@pytest.mark.parametrize("scheme", ["forward", "centred"])
+@pytest.mark.parametrize("prec,sample", [("f32", np.nan), ("f32", -np.inf), ("f64", np.inf), ("f16", 1e6)])
+def test_values_not_finite_take_single_steps(gpu, O, scheme, prec, sample):
+    """A source sample that is not finite (as the fields store it) reaches the
+    faces, and from there the flat-index neighbours in the next rows and planes,
+    where the reference has it: such a run takes single steps."""
+    room, steps, src = rooms.shoebox((28, 20, 24), seed=2), 14, (26, 18, 4)
+    recs = [(1, 3, 5), (2, 18, 4), (25, 1, 5), (13, 10, 12)]
+    pulse = rooms.gaussian_pulse(steps, 3.0)[None].copy()
+    pulse[0, 4] = sample
+    with Domain(room.dims, prec) as d:
+        d.set_scheme(scheme)
+        d.set_voxels(room.bid, room.mat, centred=scheme == "centred")
+        d.set_materials(room.admittance)
+        d.set_params()
+        d.set_sources([src], [1], pulse)
+        d.set_receivers(recs)
+        before = L.load().pfdtd_kernel_launches()
+        got, _, _ = d.run(steps)
+        assert L.load().pfdtd_kernel_launches() - before >= 2 * steps
+        P = d.download_field(L.FIELD_CURRENT)
+    pos, mat = O.encode_nodes(room.bid, room.mat, scheme == "centred")
+    want, rP, _ = O.run(pos, mat, room.dims, room.admittance, default_params(), [room.flat(*src)], [1], pulse,
+                        [room.flat(*r) for r in recs], steps, scheme=2 if scheme == "centred" else 0,
+                        double=prec == "f64", storage="f16" if prec == "f16" else None)
+    assert not np.isfinite(want).all()
+    assert np.array_equal(got, want, equal_nan=True) and np.array_equal(P, rP, equal_nan=True)
+
+
+@pytest.mark.parametrize("what", ["lambda", "material"])
+def test_rooms_that_gain_energy_take_single_steps(gpu, O, what):
+    """A lambda beyond the scheme's limit, or a material with a negative
+    admittance, may end in values that are not finite: single steps, as the
+    oracle has it to the overflow and beyond."""
+    room, steps = rooms.shoebox((20, 18, 16), seed=2), 400
+    table = room.admittance.copy()
+    params = default_params(lam=0.75 if what == "lambda" else None)
+    if what == "material":
+        table[:] = -1.2
+    src, rec, pulse = (10, 9, 8), [(3, 4, 5), (17, 2, 13)], rooms.gaussian_pulse(steps, 3.0)[None]
+    with Domain(room.dims) as d:
+        d.set_voxels(room.bid, room.mat, centred=False)
+        d.set_materials(table)
+        d.set_params(params)
+        d.set_sources([src], [1], pulse)
+        d.set_receivers(rec)
+        before = L.load().pfdtd_kernel_launches()
+        got, _, _ = d.run(steps)
+        assert L.load().pfdtd_kernel_launches() - before >= 2 * steps
+        P = d.download_field(L.FIELD_CURRENT)
+    pos, mat = O.encode_nodes(room.bid, room.mat, False)
+    want, rP, _ = O.run(pos, mat, room.dims, table, params, [room.flat(*src)], [1], pulse,
+                        [room.flat(*r) for r in rec], steps)
+    assert not np.isfinite(want).all()
+    assert np.array_equal(got, want, equal_nan=True) and np.array_equal(P, rP, equal_nan=True)
