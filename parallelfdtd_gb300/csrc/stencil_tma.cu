@@ -958,23 +958,26 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   ClassTab<A> tab{(const A*)tb, (const A*)(tb + as * d->n_classes),
                   (const A*)(tb + 2 * as * d->n_classes),
                   (const uint32_t*)(tb + 3 * as * d->n_classes), d->n_classes};
-  // Large 16-bit rooms are launched plainly: an update set up while the one
-  // before drains streams 3 % slower there than its gap costs (512 x 384 x 256:
-  // 65.1 us a step, 61.1 plainly; 512 x 384 x 200 centred BF16 74.8, 72.1), while
-  // 384 x 320 x 256 takes 43.0 against 45.5.
+  // Launched plainly are tiles of which all are resident at once: set up beside the
+  // kernel before they lie unevenly, two on one SM and none on another, or stream
+  // beside its last ones, and no second wave evens that out.  Us a step, dependent /
+  // plain: 16-bit fields in several tile columns, chunks of 20 planes and more, FP16 512 x
+  // 384 x 60 (288 CTAs of 20 planes for 304 places) 16.6 / 16.2, x 100 (33) 27.1 / 25.3, x
+  // 256 (85) 65.1 / 61.1, 1024 x 300 x 120 (304, 59) 45.2 / 44.5, BF16 centred 512 x 384 x
+  // 230 79.6 / 75.8; shorter ones gain the gap, 512 x 384 x 40 (13) 11.9 / 12.2, as do more
+  // CTAs than places, 384 x 320 x 270 (600) 44.3 / 45.2, 512 x 512 x 200 (896) 63.9 / 65.0.
+  // FP32, 4 fields of 256 x 128 x 96 (256, 47) 28.3 / 23.7, of 128^3 (32) 17.7 / 16.5, 8 of
+  // 256 x 64 x 64 17.2 / 16.0; where they fill their places only if long: 8 of 64 x 64 x
+  // 400 (288, 45) 28.3 / 24.1, FP16 8 of 192 x 192 x 128 (288, 63) 47.7 / 45.8, but 4 of 64
+  // x 64 x 400 (304, 21) 11.8 / 12.7, 8 of 64^3 (288, 7) 6.5 / 7.1.  IWB tiles, with the
+  // closure pass in between: 400 x 300 x 8 (152) 13.1 / 11.9, 96^3 (276) 13.0 / 12.6.  Single
+  // FP32 fields gain the gap at all sizes.
   const int64_t ctas = tiles * gz;
-  bool dependent = !(sizeof(S) == 2 && !BATCHED && SCHEME != 3 && d->N >= 33000000);
-  // So are tiles of which all are resident at once, but not as many as fit: set up
-  // beside the kernel before they lie unevenly, two on one SM and none on another.
-  // Us a step, dependent / plain: FP32, 4 fields of 256 x 128 x 96 (256 CTAs of 47 planes
-  // for 304 places) 28.3 / 23.7, of 128^3 (32 planes) 17.7 / 16.5, 8 of 256 x 64 x 64 17.2 /
-  // 16.0; also where they do fit, if long: 8 of 64 x 64 x 400 (288, 45) 28.3 / 24.1, FP16 8
-  // of 192 x 192 x 128 (288, 63) 47.7 / 45.8.  Shorter ones gain the gap: 4 of 64 x 64 x 400
-  // (304, 21) 11.8 / 12.7, 8 of 64^3 (288, 7) 6.5 / 7.1.  IWB tiles, with the closure pass
-  // in between: 400 x 300 x 8 (152) 13.1 / 11.9, 96^3 (276) 13.0 / 12.6; single 7-point
-  // fields gain the gap at all sizes.
+  const bool one_wave = 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident;
+  bool dependent = true;
+  if (sizeof(S) == 2 && !BATCHED && SCHEME != 3 && one_wave && gx > 1 && zc >= 20) dependent = false;
   if (SCHEME == 3 && ctas >= d->sm_count && ctas <= 2 * (int64_t)d->sm_count) dependent = false;
-  if (BATCHED && sizeof(A) == 4 && 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident &&
+  if (BATCHED && sizeof(A) == 4 && one_wave &&
       (zc >= 45 || (zc >= 16 && 10 * ctas <= 9 * resident)))
     dependent = false;
   // FP64 units bound FP64 tiles, so any unevenness costs (8 fields of 96^3 forward 162 /
