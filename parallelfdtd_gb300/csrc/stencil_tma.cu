@@ -965,7 +965,7 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // 384 x 60 (288 CTAs of 20 planes for 304 places) 16.6 / 16.2, x 100 (33) 27.1 / 25.3, x
   // 256 (85) 65.1 / 61.1, 1024 x 300 x 120 (304, 59) 45.2 / 44.5, BF16 centred 512 x 384 x
   // 230 79.6 / 75.8; shorter ones gain the gap, 512 x 384 x 40 (13) 11.9 / 12.2, as do more
-  // CTAs than places, 384 x 320 x 270 (600) 44.3 / 45.2, 512 x 512 x 200 (896) 63.9 / 65.0.
+  // CTAs than places, 512 x 512 x 200 (896) 63.9 / 65.0.
   // FP32, 4 fields of 256 x 128 x 96 (256, 47) 28.3 / 23.7, of 128^3 (32) 17.7 / 16.5, 8 of
   // 256 x 64 x 64 17.2 / 16.0; where they fill their places only if long: 8 of 64 x 64 x
   // 400 (288, 45) 28.3 / 24.1, FP16 8 of 192 x 192 x 128 (288, 63) 47.7 / 45.8, but 4 of 64
@@ -973,7 +973,9 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   // closure pass in between: 400 x 300 x 8 (152) 13.1 / 11.9, 96^3 (276) 13.0 / 12.6.  Single
   // FP32 fields gain the gap at all sizes.
   const int64_t ctas = tiles * gz;
-  const bool one_wave = 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident;
+  // (tiles of which an SM holds more than two even themselves out: 384 x 320 x 200 FP16,
+  // 600 CTAs for 608 places, 34.1 / 34.9)
+  const bool one_wave = per_sm <= 2 && 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident;
   bool dependent = true;
   if (sizeof(S) == 2 && !BATCHED && SCHEME != 3 && one_wave && gx > 1 && zc >= 20) dependent = false;
   if (SCHEME == 3 && ctas >= d->sm_count && ctas <= 2 * (int64_t)d->sm_count) dependent = false;
