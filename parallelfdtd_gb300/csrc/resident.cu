@@ -796,7 +796,8 @@ bool resident_usable(pfdtd_domain* d) {
     const bool fits = d->precision == PFDTD_F64 ? plan_bricks<double>(d, kMaxPlanes, &k, &cycles)
                                                 : plan_bricks<float>(d, kMaxPlanes, &k, &cycles);
     if (!fits) return false;
-    rs.chunk = std::max<int64_t>(2, (int64_t)(kLaunchNs / (0.7 * cycles)));
+    // (0.58 ns a cycle of the estimate at 24^3 and 64^3, 0.72 at 128^3, 0.5 in FP64)
+    rs.chunk = std::max<int64_t>(2, (int64_t)(kLaunchNs / (0.6 * cycles)));
     const int words = inbox_values(k) * (int)(d->arith_size() / 4);
     const size_t bytes = 2 * sizeof(uint64_t) * (size_t)words * k.gx * k.gy * k.gz;
     if (d->alloc(&rs.inbox, bytes) != cudaSuccess) {
