@@ -471,9 +471,10 @@ def main():
     # ---- dominant kernel alone (same stream, same arguments) ---------------
     prof_iters = 50
     k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    # (a run that stays on the SMs has not launched this kernel yet)
+    L.call("pfdtd_profile_update", d.handle, 3)
     with torch.cuda.stream(stream):
         k0.record(stream)
-    import ctypes as C
     L.call("pfdtd_profile_update", d.handle, prof_iters)
     with torch.cuda.stream(stream):
         k1.record(stream)
