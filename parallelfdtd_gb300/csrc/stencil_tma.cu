@@ -975,12 +975,15 @@ int launch_tma_t(pfdtd_domain* d, const void* cur, void* past, cudaStream_t s) {
   const int64_t ctas = tiles * gz;
   // (tiles of which an SM holds more than two even themselves out: 384 x 320 x 200 FP16,
   // 600 CTAs for 608 places, 34.1 / 34.9)
-  const bool one_wave = per_sm <= 2 && 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident;
+  // (tiles that are mostly empty weigh little: IWB 8 x 104 x 59 16.9 / 19.0)
+  const bool filled = 2 * XE >= (int64_t)gx * kTX;
+  const bool one_wave =
+      filled && per_sm <= 2 && 2 * ctas > 3 * (int64_t)d->sm_count && ctas <= resident;
   bool dependent = true;
   if (sizeof(S) == 2 && !BATCHED && SCHEME != 3 && one_wave && gx > 1 && zc >= 20) dependent = false;
-  if (SCHEME == 3 && ctas >= d->sm_count && ctas <= 2 * (int64_t)d->sm_count) dependent = false;
+  if (SCHEME == 3 && filled && ctas >= d->sm_count && ctas <= 2 * (int64_t)d->sm_count) dependent = false;
   if (BATCHED && sizeof(A) == 4 && one_wave &&
-      (zc >= 45 || (zc >= 16 && 10 * ctas <= 9 * resident)))
+      (zc >= 45 || (sizeof(S) == 4 && zc >= 16 && 10 * ctas <= 9 * resident)))
     dependent = false;
   // FP64 units bound FP64 tiles, so any unevenness costs (8 fields of 96^3 forward 162 /
   // 154, centred 287 / 245; see stencil.cu); the form without the shortcut gains the
